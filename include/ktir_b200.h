@@ -204,8 +204,12 @@ typedef struct {
     int32_t f16_arith;      /* 1: every op rounds to f16 (tile dtype f16 throughout) */
     int32_t max_is_maxnum;  /* 1: arith.maxnumf (NaN ignored), 0: maximumf */
     float max_init, sum_init;   /* the `outs` initial values of the two reductions */
+    int32_t aligned;        /* read by ktb_launch_row_softmax_any: 1: every item offset is a multiple of 8 elements */
+    int32_t reserved;
 } ktb_softmax_args;
 int ktb_launch_row_softmax(ktb_ctx* ctx, const ktb_softmax_args* args);
+/* The same for rows of any length in [1, 16384], starting at any element. */
+int ktb_launch_row_softmax_any(ktb_ctx* ctx, const ktb_softmax_args* args);
 
 /* ---- fused row programs: elementwise ops and row reductions in one pass over HBM ----------
  * A statement whose value mixes elementwise ops with reductions along the last tile dimension — layer

@@ -21,6 +21,25 @@ static __device__ __forceinline__ float sm_comb(float a, float b) {
     return R16 ? ktb_round16(r) : r;
 }
 
+// How a row of any length is dealt out: whole warps, `nv` chunks of 8 elements per thread.  The fewest warps that hold
+// the row (and the partial chunks at its two ends) with `max_nv` chunks per thread, then as few chunks as those need;
+// rows of one warp share a CTA of 256 threads eight at a time and need no block barrier, rows of two warps four at
+// a time.  With less than 512 threads per SM from all rows together a row gets more threads, which shortens its chain.
+struct rg_split {
+    int threads, nv, groups;
+};
+static inline rg_split rg_choose(int cols, bool aligned, int64_t rows, int sm_count, int max_nv, int max_threads) {
+    const int vecs = (cols + (aligned ? 7 : 14)) / 8;
+    rg_split s;
+    int nv = max_nv;
+    auto threads = [&](int n) { return (vecs + 32 * n - 1) / (32 * n) * 32; };
+    while (nv > 1 && rows * threads(nv) < (int64_t)sm_count * 512 && threads(nv / 2) <= max_threads) nv /= 2;
+    s.threads = threads(nv);
+    s.nv = (vecs + s.threads - 1) / s.threads;
+    s.groups = s.threads == 32 ? 8 : 256 / s.threads > 4 ? 4 : 256 / s.threads < 1 ? 1 : 256 / s.threads;
+    return s;
+}
+
 // Named barrier of one row group (ids 1..4 as literals so only those are reserved).
 static __device__ __forceinline__ void group_barrier(int id, int threads) {
     switch (id) {
@@ -105,6 +124,153 @@ static __device__ __forceinline__ float row_fold(const float (&x)[NV][8], int T,
     return __shfl_sync(0xffffffffu, v[0], 0, w);
 }
 
+
+// ---- rows of any length ---------------------------------------------------------------------------------
+static __device__ __forceinline__ void rg_barrier(int group, int T) {
+    if (T == 32) __syncwarp();
+    else group_barrier(1 + group, T);
+}
+
+// A row that starts `mis` elements (0..7) after a boundary of 8 is walked in the memory's own 8-element chunks: chunk
+// c holds elements 8 c - mis ... 8 c - mis + 7, of which the first and the last chunk may have fewer.  Whole chunks
+// move as 16-byte vectors whatever the row's start; only the elements of the edge chunks go one by one.
+static __device__ __forceinline__ bool rg_whole(int c, int mis, int cols) { return c * 8 >= mis && c * 8 - mis + 8 <= cols; }
+static __device__ __forceinline__ bool rg_any(int c, int mis, int cols) { return c * 8 - mis < cols; }
+
+// Chunk c of an f16 row as packed halves; what lies outside the row keeps what `raw` held.
+static __device__ __forceinline__ void rg_load_h(const __half* row, int mis, int cols, int c, uint4& raw) {
+    const __half* p = row + (c * 8 - mis);
+    if (rg_whole(c, mis, cols)) {
+        raw = __ldcs(reinterpret_cast<const uint4*>(p));
+    } else if (rg_any(c, mis, cols)) {
+        __half* e = reinterpret_cast<__half*>(&raw);
+#pragma unroll
+        for (int v = 0; v < 8; ++v)
+            if (c * 8 + v >= mis && c * 8 + v - mis < cols) e[v] = p[v];
+    }
+}
+// `same`: the destination row starts at the same offset from a boundary as the row whose chunks these are.
+static __device__ __forceinline__ void rg_store_h(__half* row, int mis, int cols, int c, bool same, const uint4& raw) {
+    __half* p = row + (c * 8 - mis);
+    if (same && rg_whole(c, mis, cols)) {
+        __stcs(reinterpret_cast<uint4*>(p), raw);
+    } else if (rg_any(c, mis, cols)) {
+        const __half* e = reinterpret_cast<const __half*>(&raw);
+#pragma unroll
+        for (int v = 0; v < 8; ++v)
+            if (c * 8 + v >= mis && c * 8 + v - mis < cols) p[v] = e[v];
+    }
+}
+// The same as f32 values for an f16 or f32 tile whose row starts at element `off`; `same` as above (a weight row,
+// say, may start elsewhere).
+static __device__ __forceinline__ void rg_load8(const void* arena, int64_t off, int dtype, int mis, int cols, int c, bool same,
+                                                float (&x)[8]) {
+    const int64_t at = off + (c * 8 - mis);
+    if (same && rg_whole(c, mis, cols)) {
+        if (dtype == KTB_F16) {
+            const uint4 raw = *reinterpret_cast<const uint4*>(reinterpret_cast<const __half*>(arena) + at);
+            const __half2* h = reinterpret_cast<const __half2*>(&raw);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float2 f = __half22float2(h[i]);
+                x[2 * i] = f.x;
+                x[2 * i + 1] = f.y;
+            }
+        } else {
+            const float4 lo = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(arena) + at);
+            const float4 hi = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(arena) + at + 4);
+            x[0] = lo.x; x[1] = lo.y; x[2] = lo.z; x[3] = lo.w;
+            x[4] = hi.x; x[5] = hi.y; x[6] = hi.z; x[7] = hi.w;
+        }
+    } else if (rg_any(c, mis, cols)) {
+#pragma unroll
+        for (int v = 0; v < 8; ++v)
+            if (c * 8 + v >= mis && c * 8 + v - mis < cols)
+                x[v] = dtype == KTB_F16 ? __half2float(reinterpret_cast<const __half*>(arena)[at + v])
+                                        : reinterpret_cast<const float*>(arena)[at + v];
+    }
+}
+static __device__ __forceinline__ void rg_store8(void* arena, int64_t off, int dtype, int mis, int cols, int c, bool same,
+                                                 const float (&x)[8]) {
+    if (dtype == KTB_F16) {
+        uint4 raw;
+        __half2* h = reinterpret_cast<__half2*>(&raw);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) h[i] = __floats2half2_rn(x[2 * i], x[2 * i + 1]);
+        rg_store_h(reinterpret_cast<__half*>(arena) + off, mis, cols, c, same, raw);
+        return;
+    }
+    float* p = reinterpret_cast<float*>(arena) + off + (c * 8 - mis);
+    if (same && rg_whole(c, mis, cols)) {
+        __stcs(reinterpret_cast<float4*>(p), make_float4(x[0], x[1], x[2], x[3]));
+        __stcs(reinterpret_cast<float4*>(p + 4), make_float4(x[4], x[5], x[6], x[7]));
+    } else if (rg_any(c, mis, cols)) {
+#pragma unroll
+        for (int v = 0; v < 8; ++v)
+            if (c * 8 + v >= mis && c * 8 + v - mis < cols) p[v] = x[v];
+    }
+}
+// Chunk c of the values to be folded, to shared memory; the row then begins at buf + mis.
+static __device__ __forceinline__ void rg_park8(float* buf, int mis, int cols, int c, const float (&x)[8]) {
+    if (!rg_any(c, mis, cols)) return;
+    reinterpret_cast<float4*>(buf + c * 8)[0] = make_float4(x[0], x[1], x[2], x[3]);
+    reinterpret_cast<float4*>(buf + c * 8)[1] = make_float4(x[4], x[5], x[6], x[7]);
+}
+
+// Three levels of the reference's fold at once: of n values, level one leaves n - n / 2 — value i is x[i] (op)
+// x[i + n / 2], and an odd last one is carried along (ktir_cpu/dialects/linalg_ops.py:86-133).
+template <int OP, bool MAXNUM, bool R16>
+static __device__ __forceinline__ float rg_level3(const float* x, int n, int i) {
+    const int h0 = n >> 1, n1 = n - h0, h1 = n1 >> 1, n2 = n1 - h1, h2 = n2 >> 1;
+    auto l1 = [&](int k) { return k < h0 ? sm_comb<OP, MAXNUM, R16>(x[k], x[k + h0]) : x[k + h0]; };
+    auto l2 = [&](int k) { return k < h1 ? sm_comb<OP, MAXNUM, R16>(l1(k), l1(k + h1)) : l1(k + h1); };
+    return i < h2 ? sm_comb<OP, MAXNUM, R16>(l2(i), l2(i + h2)) : l2(i + h2);
+}
+static __host__ __device__ __forceinline__ int rg_after3(int n) {
+    n -= n >> 1;
+    n -= n >> 1;
+    return n - (n >> 1);
+}
+
+// Floats of shared memory one row needs for rg_fold: the chunks of values, an eighth of them, the result.
+static __host__ __device__ __forceinline__ int rg_chunk_floats(int cols) { return (cols + 14) & ~7; }
+static __host__ __device__ __forceinline__ int rg_scratch(int cols) {
+    return rg_chunk_floats(cols) + ((rg_after3(cols) + 3) & ~3) + 4;
+}
+
+// Fold of the `cols` values at buf + mis that the T threads of the group have written there, in the reference's order
+// for any length; every thread gets the result.  Three levels per barrier (the values cross shared memory once and an
+// eighth of them again); the last 32 by shuffles in the first warp.
+template <int OP, bool MAXNUM, bool R16>
+static __device__ __forceinline__ float rg_fold(float* buf, int mis, int cols, int T, int t, int group) {
+    float* src = buf + mis;
+    float* dst = buf + rg_chunk_floats(cols);
+    float* result = dst + ((rg_after3(cols) + 3) & ~3);
+    rg_barrier(group, T);
+    int n = cols;
+    while (n > 256) {
+        const int m = rg_after3(n);
+        for (int i = t; i < m; i += T) dst[i] = rg_level3<OP, MAXNUM, R16>(src, n, i);
+        rg_barrier(group, T);
+        float* o = src;
+        src = dst;
+        dst = o;
+        n = m;
+    }
+    if (t < 32) {
+        const int m = rg_after3(n);
+        float v = t < m ? rg_level3<OP, MAXNUM, R16>(src, n, t) : 0.f;
+        for (n = m; n > 1;) {
+            const int h = n >> 1;
+            const float o = __shfl_down_sync(0xffffffffu, v, h);
+            v = t < h ? sm_comb<OP, MAXNUM, R16>(v, o) : o;
+            n -= h;
+        }
+        if (t == 0) *result = v;
+    }
+    rg_barrier(group, T);
+    return *result;
+}
 
 // The same fold of a sum whose every add rounds to f16, on packed halves: an f16 add of two f16 values is
 // the f32 add rounded to f16 (24 >= 2 * 11 + 2 significand bits: the double rounding cannot show), so the

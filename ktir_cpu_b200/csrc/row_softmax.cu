@@ -15,6 +15,7 @@
 #include <stdlib.h>
 
 #include "row_fold.cuh"
+#include "vm.cuh"
 
 static __device__ __forceinline__ float sm_ex2(float x) {
     float y;
@@ -351,4 +352,235 @@ extern "C" int ktb_launch_row_softmax(ktb_ctx* ctx, const ktb_softmax_args* args
     }
     KTB_CHECK_LAUNCH(ctx, "ktb_row_softmax_kernel");
     return KTB_OK;
+}
+
+// ---- rows of any length and alignment -----------------------------------------------------------------
+// One pass over HBM for rows that are no power of two long, or whose start is not 16-byte aligned (row_fold.cuh: how a
+// row is cut into chunks and dealt out).  This form keeps the row as f32 values.  f16 arithmetic has the reference's
+// rounding points and its order of the sum (rg_fold); otherwise max and sum are taken by shuffles, expf and the
+// division are those of the step-by-step form.  f16[4096, 3000], f16 arithmetic: 39.0 us (37 steps before).
+template <int NV, bool R16, bool MAXNUM>
+__global__ void __launch_bounds__(512) ktb_row_softmax_any_kernel(const ktb_softmax_args a, int T, int64_t total_rows) {
+    extern __shared__ float rg_smem[];
+    const int group = threadIdx.x / T;
+    const int t = threadIdx.x - group * T;
+    const int64_t row = (int64_t)blockIdx.x * (blockDim.x / T) + group;
+    if (row >= total_rows) return;                       // whole row groups: the barriers are per group
+    float* buf = rg_smem + group * (R16 ? rg_scratch(a.cols) : 32);
+    const int lane = threadIdx.x & 31, warp = t >> 5, warps = T >> 5;
+    const int64_t item = (uint32_t)row / (uint32_t)a.rows_per_item;
+    const int64_t r = row - item * a.rows_per_item;
+    const int64_t in_off = a.dev_item_offsets[item * 2] + r * a.in_row_stride;
+    const int64_t out_off = a.dev_item_offsets[item * 2 + 1] + r * a.out_row_stride;
+    const int cols = a.cols, mis = (int)(in_off & 7);
+    const bool same = ((in_off ^ out_off) & 7) == 0;
+
+    float x[NV][8];
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+#pragma unroll
+        for (int v = 0; v < 8; ++v) x[j][v] = -INFINITY;
+        rg_load8(a.arena, in_off, a.in_dtype, mis, cols, j * T + t, true, x[j]);
+    }
+    float mx = x[0][0];
+#pragma unroll
+    for (int j = 0; j < NV; ++j)
+#pragma unroll
+        for (int v = 0; v < 8; ++v) mx = sm_max<MAXNUM>(mx, x[j][v]);
+#pragma unroll
+    for (int d = 16; d >= 1; d >>= 1) mx = sm_max<MAXNUM>(mx, __shfl_xor_sync(0xffffffffu, mx, d));
+    if (warps > 1) {
+        if (lane == 0) buf[warp] = mx;
+        rg_barrier(group, T);
+        mx = buf[0];
+        for (int k = 1; k < warps; ++k) mx = sm_max<MAXNUM>(mx, buf[k]);
+    }
+    mx = sm_max<MAXNUM>(mx, a.max_init);
+
+    float sum = 0.f;
+    if (R16) {
+        if (warps > 1) rg_barrier(group, T);             // the per-warp maxima have been read
+#pragma unroll
+        for (int j = 0; j < NV; ++j) {
+#pragma unroll
+            for (int v = 0; v < 8; ++v) x[j][v] = ktb_round16(expf(ktb_round16(x[j][v] - mx)));
+            rg_park8(buf, mis, cols, j * T + t, x[j]);
+        }
+        sum = ktb_round16(rg_fold<1, MAXNUM, true>(buf, mis, cols, T, t, group) + a.sum_init);
+    } else {
+        float s0 = 0.f, s1 = 0.f;                        // (lanes outside the row hold -inf and add nothing)
+#pragma unroll
+        for (int j = 0; j < NV; ++j)
+#pragma unroll
+            for (int v = 0; v < 8; ++v) {
+                x[j][v] = expf(x[j][v] - mx);
+                if (v & 1) s1 += x[j][v];
+                else s0 += x[j][v];
+            }
+        sum = s0 + s1;
+#pragma unroll
+        for (int d = 16; d >= 1; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+        if (warps > 1) {
+            if (lane == 0) buf[16 + warp] = sum;
+            rg_barrier(group, T);
+            sum = buf[16];
+            for (int k = 1; k < warps; ++k) sum += buf[16 + k];
+        }
+        sum = sum + a.sum_init;
+    }
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+#pragma unroll
+        for (int v = 0; v < 8; ++v) x[j][v] = x[j][v] / sum;
+        rg_store8(a.arena, out_off, a.out_dtype, mis, cols, j * T + t, same, x[j]);
+    }
+}
+
+// f16 rows with f32 statistics and f16 results, the common case: the row stays in registers as packed f16 (NV x 4
+// registers) and the exponential is evaluated twice, once for the sum and once for the result, so nothing is rounded
+// on the way.  The exponent is one fma per element, x * log2e - max * log2e: the rounding of max * log2e is common to
+// the row and cancels in the quotient.  Lanes past the ends of the row hold -inf and add nothing.  Bound by the
+// latency of a row's chain and HBM together.  f16[4096, 3000]: 763 us in 39 steps over f32 copies of the tile, 20.7 us
+// with the row as f32 values (half the resident rows), 14.4 us here (7.6 at the measured copy rate);
+// 3001 columns 16.5 us (41.2 us when every element was loaded and stored by itself).
+template <int NV, bool MAXNUM>
+__global__ void __launch_bounds__(256, NV > 4 ? 4 : 6)
+ktb_row_softmax_any_h_kernel(const ktb_softmax_args a, int T, int64_t total_rows) {
+    __shared__ float xmax[8], xsum[8];                   // one slot per warp of the CTA
+    const int group = threadIdx.x / T;
+    const int t = threadIdx.x - group * T;
+    const int64_t row = (int64_t)blockIdx.x * (blockDim.x / T) + group;
+    if (row >= total_rows) return;                       // whole row groups: the barriers are per group
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, w0 = group * (T >> 5), warps = T >> 5;
+    const int64_t item = (uint32_t)row / (uint32_t)a.rows_per_item;
+    const int64_t r = row - item * a.rows_per_item;
+    const int64_t in_off = a.dev_item_offsets[item * 2] + r * a.in_row_stride;
+    const int64_t out_off = a.dev_item_offsets[item * 2 + 1] + r * a.out_row_stride;
+    const __half* src = reinterpret_cast<const __half*>(a.arena) + in_off;
+    __half* dst = reinterpret_cast<__half*>(a.arena) + out_off;
+    const int cols = a.cols, mis = (int)(in_off & 7);
+    const bool same = ((in_off ^ out_off) & 7) == 0;
+
+    uint4 raw[NV];
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        raw[j] = make_uint4(0xfc00fc00u, 0xfc00fc00u, 0xfc00fc00u, 0xfc00fc00u);      // -inf
+        rg_load_h(src, mis, cols, j * T + t, raw[j]);
+    }
+    __half2 m2 = *reinterpret_cast<const __half2*>(&raw[0].x);
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        const __half2* h = reinterpret_cast<const __half2*>(&raw[j]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) m2 = MAXNUM ? __hmax2(m2, h[i]) : __hmax2_nan(m2, h[i]);
+    }
+#pragma unroll
+    for (int d = 16; d >= 1; d >>= 1) {
+        const uint32_t o = __shfl_xor_sync(0xffffffffu, *reinterpret_cast<uint32_t*>(&m2), d);
+        const __half2 oh = *reinterpret_cast<const __half2*>(&o);
+        m2 = MAXNUM ? __hmax2(m2, oh) : __hmax2_nan(m2, oh);
+    }
+    float mx = sm_max<MAXNUM>(__low2float(m2), __high2float(m2));
+    if (warps > 1) {
+        if (lane == 0) xmax[warp] = mx;
+        group_barrier(1 + group, T);
+        mx = xmax[w0];
+        for (int k = 1; k < warps; ++k) mx = sm_max<MAXNUM>(mx, xmax[w0 + k]);
+    }
+    mx = sm_max<MAXNUM>(mx, a.max_init);
+    const float mxs = -mx * 1.4426950408889634f;
+    const uint64_t l2e2 = sm_pack2(1.4426950408889634f, 1.4426950408889634f), negm2 = sm_pack2(mxs, mxs);
+    auto exp2of = [&](__half2 h, float& p0, float& p1) {
+        const float2 f = __half22float2(h);
+        sm_unpack2(sm_fma2(sm_pack2(f.x, f.y), l2e2, negm2), p0, p1);
+        p0 = sm_ex2(p0);
+        p1 = sm_ex2(p1);
+    };
+    uint64_t acc0 = sm_pack2(0.f, 0.f), acc1 = acc0;
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        const __half2* h = reinterpret_cast<const __half2*>(&raw[j]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float p0, p1;
+            exp2of(h[i], p0, p1);
+            if (i & 1) acc1 = sm_add2(acc1, sm_pack2(p0, p1));
+            else acc0 = sm_add2(acc0, sm_pack2(p0, p1));
+        }
+    }
+    float a0, a1, b0, b1;
+    sm_unpack2(acc0, a0, a1);
+    sm_unpack2(acc1, b0, b1);
+    float sum = (a0 + a1) + (b0 + b1);
+#pragma unroll
+    for (int d = 16; d >= 1; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+    if (warps > 1) {
+        if (lane == 0) xsum[warp] = sum;
+        group_barrier(1 + group, T);
+        sum = xsum[w0];
+        for (int k = 1; k < warps; ++k) sum += xsum[w0 + k];
+    }
+    const float inv = 1.0f / (sum + a.sum_init);
+    // (opaque to the optimiser, which otherwise keeps the exponentials of the first evaluation alive)
+#pragma unroll
+    for (int j = 0; j < NV; ++j)
+        asm volatile("" : "+r"(raw[j].x), "+r"(raw[j].y), "+r"(raw[j].z), "+r"(raw[j].w));
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        const __half2* h = reinterpret_cast<const __half2*>(&raw[j]);
+        uint4 o;
+        __half2* ho = reinterpret_cast<__half2*>(&o);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float p0, p1;
+            exp2of(h[i], p0, p1);
+            ho[i] = __floats2half2_rn(p0 * inv, p1 * inv);
+        }
+        rg_store_h(dst, mis, cols, j * T + t, same, o);
+    }
+}
+
+template <int NV>
+static int launch_softmax_any(ktb_ctx* ctx, const ktb_softmax_args& a, const rg_split& s, int64_t total_rows) {
+    const unsigned blocks = (unsigned)((total_rows + s.groups - 1) / s.groups), threads = s.threads * s.groups;
+    const bool mn = a.max_is_maxnum != 0, r16 = a.f16_arith != 0;
+    if (a.in_dtype == KTB_F16 && a.out_dtype == KTB_F16 && !r16) {
+        if (mn) ktb_row_softmax_any_h_kernel<NV, true><<<blocks, threads, 0, ctx->stream>>>(a, s.threads, total_rows);
+        else ktb_row_softmax_any_h_kernel<NV, false><<<blocks, threads, 0, ctx->stream>>>(a, s.threads, total_rows);
+    } else if constexpr (NV <= 4) {
+        const size_t smem = (r16 ? rg_scratch(a.cols) : 32) * sizeof(float) * s.groups;
+        auto k = r16 ? (mn ? ktb_row_softmax_any_kernel<NV, true, true> : ktb_row_softmax_any_kernel<NV, true, false>)
+                     : (mn ? ktb_row_softmax_any_kernel<NV, false, true> : ktb_row_softmax_any_kernel<NV, false, false>);
+        if (smem > 48 * 1024) KTB_CUDA(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        k<<<blocks, threads, smem, ctx->stream>>>(a, s.threads, total_rows);
+    }
+    KTB_CHECK_LAUNCH(ctx, "ktb_row_softmax_any_kernel");
+    return KTB_OK;
+}
+
+extern "C" int ktb_launch_row_softmax_any(ktb_ctx* ctx, const ktb_softmax_args* args) {
+    if (!ctx || !args) return KTB_E_ARG;
+    const ktb_softmax_args& a = *args;
+    if (a.n_items <= 0 || a.rows_per_item <= 0) return KTB_OK;
+    // (rows that start between boundaries have a partial chunk at either end; 2048 chunks are what 512 threads hold)
+    const bool aligned = a.aligned && a.in_row_stride % 8 == 0;
+    if (a.cols < 1 || a.cols > (aligned ? 16384 : 16377))
+        return ktb_fail(ctx, KTB_E_UNSUPPORTED, "row_softmax_any", "cols must lie in [1, 16384] (16377 for unaligned rows)");
+    if ((a.in_dtype != KTB_F16 && a.in_dtype != KTB_F32) || (a.out_dtype != KTB_F16 && a.out_dtype != KTB_F32))
+        return ktb_fail(ctx, KTB_E_UNSUPPORTED, "row_softmax_any", "dtype must be f16 or f32");
+    const int64_t total_rows = a.n_items * (int64_t)a.rows_per_item;
+    if (total_rows >= (1ll << 31)) return ktb_fail(ctx, KTB_E_UNSUPPORTED, "row_softmax_any", "more than 2^31 rows");
+    // packed halves: up to 8 chunks per thread (128 bytes in flight each), f32 values: up to 4
+    const bool packed = a.in_dtype == KTB_F16 && a.out_dtype == KTB_F16 && !a.f16_arith;
+    const rg_split s = rg_choose(a.cols, aligned, total_rows, ctx->sm_count, packed ? 8 : 4, packed ? 256 : 512);
+    switch (s.nv) {
+        case 1: return launch_softmax_any<1>(ctx, a, s, total_rows);
+        case 2: return launch_softmax_any<2>(ctx, a, s, total_rows);
+        case 3: return launch_softmax_any<3>(ctx, a, s, total_rows);
+        case 4: return launch_softmax_any<4>(ctx, a, s, total_rows);
+        case 5: return launch_softmax_any<5>(ctx, a, s, total_rows);
+        case 6: return launch_softmax_any<6>(ctx, a, s, total_rows);
+        case 7: return launch_softmax_any<7>(ctx, a, s, total_rows);
+        default: return launch_softmax_any<8>(ctx, a, s, total_rows);
+    }
 }

@@ -80,7 +80,7 @@ class SoftmaxArgs(C.Structure):
                 ("in_row_stride", C.c_int64), ("out_row_stride", C.c_int64),
                 ("in_dtype", C.c_int32), ("out_dtype", C.c_int32),
                 ("f16_arith", C.c_int32), ("max_is_maxnum", C.c_int32),
-                ("max_init", C.c_float), ("sum_init", C.c_float)]
+                ("max_init", C.c_float), ("sum_init", C.c_float), ("aligned", C.c_int32), ("reserved", C.c_int32)]
 
 
 ROWS_MAX_IN = 3
@@ -190,6 +190,7 @@ SYMBOLS = {
     "ktb_launch_ew_stream": (C.c_int, [C.c_void_p, C.POINTER(EwArgs)]),
     "ktb_launch_row_program": (C.c_int, [C.c_void_p, C.POINTER(RowProgArgs)]),
     "ktb_launch_row_softmax": (C.c_int, [C.c_void_p, C.POINTER(SoftmaxArgs)]),
+    "ktb_launch_row_softmax_any": (C.c_int, [C.c_void_p, C.POINTER(SoftmaxArgs)]),
     "ktb_launch_rows_program": (C.c_int, [C.c_void_p, C.POINTER(RowsArgs)]),
     "ktb_launch_scatter_rows": (C.c_int, [C.c_void_p, C.POINTER(RowsArgs)]),
     "ktb_scatter_scratch_bytes": (C.c_size_t, [C.c_int64, C.c_int64]),
