@@ -276,6 +276,8 @@ typedef struct {
     ktb_rp_side side[KTB_RP_MAX_SIDE];
 } ktb_rowprog_args;
 int ktb_launch_row_program(ktb_ctx* ctx, const ktb_rowprog_args* args);
+/* The same for rows of any length in [1, 16384]; offsets and strides are any number of elements. */
+int ktb_launch_row_program_any(ktb_ctx* ctx, const ktb_rowprog_args* args);
 
 /* ---- row gather / ordered row scatter ---------------------------------------------
  * A statement moves E = n_tiles * tile_rows rows ("entries") of `cols` elements per

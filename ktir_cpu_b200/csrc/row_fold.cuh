@@ -149,6 +149,14 @@ static __device__ __forceinline__ void rg_load_h(const __half* row, int mis, int
             if (c * 8 + v >= mis && c * 8 + v - mis < cols) e[v] = p[v];
     }
 }
+// ... of a row whose own start lies elsewhere between boundaries than `mis` (chunks laid out for another row).
+static __device__ __forceinline__ void rg_load_h_apart(const __half* row, int mis, int cols, int c, uint4& raw) {
+    const __half* p = row + (c * 8 - mis);
+    __half* e = reinterpret_cast<__half*>(&raw);
+#pragma unroll
+    for (int v = 0; v < 8; ++v)
+        if (c * 8 + v >= mis && c * 8 + v - mis < cols) e[v] = p[v];
+}
 // `same`: the destination row starts at the same offset from a boundary as the row whose chunks these are.
 static __device__ __forceinline__ void rg_store_h(__half* row, int mis, int cols, int c, bool same, const uint4& raw) {
     __half* p = row + (c * 8 - mis);
@@ -217,12 +225,12 @@ static __device__ __forceinline__ void rg_park8(float* buf, int mis, int cols, i
     reinterpret_cast<float4*>(buf + c * 8)[1] = make_float4(x[4], x[5], x[6], x[7]);
 }
 
-// Three levels of the reference's fold at once: of n values, level one leaves n - n / 2 — value i is x[i] (op)
-// x[i + n / 2], and an odd last one is carried along (ktir_cpu/dialects/linalg_ops.py:86-133).
-template <int OP, bool MAXNUM, bool R16>
-static __device__ __forceinline__ float rg_level3(const float* x, int n, int i) {
+// Three levels of the reference's fold at once: of n values, level one leaves n - n / 2 — value i is x(i) (op)
+// x(i + n / 2), and an odd last one is carried along (ktir_cpu/dialects/linalg_ops.py:86-133).
+template <int OP, bool MAXNUM, bool R16, typename F>
+static __device__ __forceinline__ float rg_level3(F x, int n, int i) {
     const int h0 = n >> 1, n1 = n - h0, h1 = n1 >> 1, n2 = n1 - h1, h2 = n2 >> 1;
-    auto l1 = [&](int k) { return k < h0 ? sm_comb<OP, MAXNUM, R16>(x[k], x[k + h0]) : x[k + h0]; };
+    auto l1 = [&](int k) { return k < h0 ? sm_comb<OP, MAXNUM, R16>(x(k), x(k + h0)) : x(k + h0); };
     auto l2 = [&](int k) { return k < h1 ? sm_comb<OP, MAXNUM, R16>(l1(k), l1(k + h1)) : l1(k + h1); };
     return i < h2 ? sm_comb<OP, MAXNUM, R16>(l2(i), l2(i + h2)) : l2(i + h2);
 }
@@ -232,35 +240,46 @@ static __host__ __device__ __forceinline__ int rg_after3(int n) {
     return n - (n >> 1);
 }
 
-// Floats of shared memory one row needs for rg_fold: the chunks of values, an eighth of them, the result.
-static __host__ __device__ __forceinline__ int rg_chunk_floats(int cols) { return (cols + 14) & ~7; }
-static __host__ __device__ __forceinline__ int rg_scratch(int cols) {
-    return rg_chunk_floats(cols) + ((rg_after3(cols) + 3) & ~3) + 4;
+// Elements (of the row's dtype, or floats) that the chunks of a row take in shared memory, and the floats that its fold
+// takes beside them: an eighth of the values, an eighth of those, the result.
+static __host__ __device__ __forceinline__ int rg_chunk_elems(int cols) { return (cols + 14) & ~7; }
+static __host__ __device__ __forceinline__ int rg_fold_floats(int cols) {
+    const int n1 = rg_after3(cols);
+    return ((n1 + 3) & ~3) + ((rg_after3(n1) + 3) & ~3) + 4;
 }
 
-// Fold of the `cols` values at buf + mis that the T threads of the group have written there, in the reference's order
-// for any length; every thread gets the result.  Three levels per barrier (the values cross shared memory once and an
-// eighth of them again); the last 32 by shuffles in the first warp.
-template <int OP, bool MAXNUM, bool R16>
-static __device__ __forceinline__ float rg_fold(float* buf, int mis, int cols, int T, int t, int group) {
-    float* src = buf + mis;
-    float* dst = buf + rg_chunk_floats(cols);
-    float* result = dst + ((rg_after3(cols) + 3) & ~3);
+// Fold of value(0) .. value(cols - 1), which the T threads of the group have put where `value` finds them, in the
+// reference's order for any length; every thread gets the result, and what `value` reads is left alone.  Three levels
+// per barrier (every value is read once, an eighth of that again); the last 32 by shuffles in the first warp.
+template <int OP, bool MAXNUM, bool R16, typename F>
+static __device__ __forceinline__ float rg_fold(F value, float* tmp, int cols, int T, int t, int group) {
+    float* dst = tmp;
+    float* other = tmp + ((rg_after3(cols) + 3) & ~3);
+    float* result = tmp + rg_fold_floats(cols) - 4;
     rg_barrier(group, T);
     int n = cols;
-    while (n > 256) {
+    float v = 0.f;
+    if (n > 256) {
         const int m = rg_after3(n);
-        for (int i = t; i < m; i += T) dst[i] = rg_level3<OP, MAXNUM, R16>(src, n, i);
-        rg_barrier(group, T);
-        float* o = src;
-        src = dst;
-        dst = o;
+        for (int i = t; i < m; i += T) dst[i] = rg_level3<OP, MAXNUM, R16>(value, n, i);
         n = m;
+        rg_barrier(group, T);
+        while (n > 256) {
+            const int k = rg_after3(n);
+            const float* src = dst;
+            for (int i = t; i < k; i += T) other[i] = rg_level3<OP, MAXNUM, R16>([&](int q) { return src[q]; }, n, i);
+            rg_barrier(group, T);
+            float* o = dst;
+            dst = other;
+            other = o;
+            n = k;
+        }
+        if (t < 32 && t < rg_after3(n)) v = rg_level3<OP, MAXNUM, R16>([&](int q) { return dst[q]; }, n, t);
+    } else if (t < 32 && t < rg_after3(n)) {
+        v = rg_level3<OP, MAXNUM, R16>(value, n, t);
     }
     if (t < 32) {
-        const int m = rg_after3(n);
-        float v = t < m ? rg_level3<OP, MAXNUM, R16>(src, n, t) : 0.f;
-        for (n = m; n > 1;) {
+        for (n = rg_after3(n); n > 1;) {
             const int h = n >> 1;
             const float o = __shfl_down_sync(0xffffffffu, v, h);
             v = t < h ? sm_comb<OP, MAXNUM, R16>(v, o) : o;

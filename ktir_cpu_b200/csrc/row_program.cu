@@ -724,6 +724,8 @@ ktb_row_norm_h_kernel(const __grid_constant__ ktb_rowprog_args a, const rp_norm 
     }
 }
 
+#include "row_program_any.cuh"
+
 template <int NB, int NV>
 static void rp_launch_norm_blocks(ktb_ctx* ctx, const ktb_rowprog_args& a, const rp_norm& m, int T, int64_t total_rows) {
     const int groups = 256 / T;
@@ -788,25 +790,25 @@ static int rp_check_program(ktb_ctx* ctx, const ktb_vm_program& p, int n_in, boo
     return KTB_OK;
 }
 
-extern "C" int ktb_launch_row_program(ktb_ctx* ctx, const ktb_rowprog_args* args) {
-    if (!ctx || !args) return KTB_E_ARG;
-    const ktb_rowprog_args& a = *args;
-    if (a.n_items <= 0 || a.rows_per_item <= 0) return KTB_OK;
+// What both launchers check; `any`: rows of any length, at any element.
+static int rp_check_args(ktb_ctx* ctx, const ktb_rowprog_args& a, bool any) {
     if (a.n_in < 1 || a.n_in > KTB_VM_MAX_IN || a.n_red < 0 || a.n_red > KTB_RP_MAX_RED || a.n_scal < 0 ||
         a.n_scal > KTB_RP_MAX_SCAL || a.n_in + a.n_scal > KTB_VM_REGS)
         return ktb_fail(ctx, KTB_E_ARG, "row_program", "bad operand / phase counts");
-    if (a.cols < 8 || a.cols > 16384 || (a.cols & (a.cols - 1)) != 0)
+    if (any && (a.cols < 1 || a.cols > 16384))
+        return ktb_fail(ctx, KTB_E_UNSUPPORTED, "row_program", "cols must lie in [1, 16384]");
+    if (!any && (a.cols < 8 || a.cols > 16384 || (a.cols & (a.cols - 1)) != 0))
         return ktb_fail(ctx, KTB_E_UNSUPPORTED, "row_program", "cols must be a power of two in [8, 16384]");
     bool any_blocked = a.out.blocked != 0;
     for (int p = 0; p < a.n_red; ++p) any_blocked = any_blocked || a.red[p].blocked;
     if (a.n_blocks < 1 || a.n_blocks > 4096 || (!any_blocked && a.n_blocks != 1) || (a.out.blocked && a.out_per_row))
         return ktb_fail(ctx, KTB_E_ARG, "row_program", "bad column-block count");
-    for (int k = 0; any_blocked && k <= a.n_in; ++k)
+    for (int k = 0; !any && any_blocked && k <= a.n_in; ++k)
         if (a.blk_stride[k] % 8) return ktb_fail(ctx, KTB_E_UNSUPPORTED, "row_program", "block strides must be multiples of 8 elements");
     for (int k = 0; k <= a.n_in; ++k) {
         if (a.dtype[k] != KTB_F16 && a.dtype[k] != KTB_F32)
             return ktb_fail(ctx, KTB_E_UNSUPPORTED, "row_program", "operand dtype must be f16 or f32");
-        if (a.row_stride[k] % 8 && !(k == a.n_in && a.out_per_row))
+        if (!any && a.row_stride[k] % 8 && !(k == a.n_in && a.out_per_row))
             return ktb_fail(ctx, KTB_E_UNSUPPORTED, "row_program", "row strides must be multiples of 8 elements");
     }
     if (a.n_side < 0 || a.n_side > KTB_RP_MAX_SIDE || (a.n_side && a.out_per_row))
@@ -828,6 +830,28 @@ extern "C" int ktb_launch_row_program(ktb_ctx* ctx, const ktb_rowprog_args* args
         if (a.scal[s].ready_after < -1 || a.scal[s].ready_after >= a.n_red || (s && a.scal[s].ready_after < a.scal[s - 1].ready_after))
             return ktb_fail(ctx, KTB_E_ARG, "row_program", "row scalars must be sorted by the last reduction they read");
     }
+    if (a.n_items * (int64_t)a.rows_per_item >= (1ll << 31))
+        return ktb_fail(ctx, KTB_E_UNSUPPORTED, "row_program", "more than 2^31 rows");
+    return KTB_OK;
+}
+
+extern "C" int ktb_launch_row_program_any(ktb_ctx* ctx, const ktb_rowprog_args* args) {
+    if (!ctx || !args) return KTB_E_ARG;
+    const ktb_rowprog_args& a = *args;
+    if (a.n_items <= 0 || a.rows_per_item <= 0) return KTB_OK;
+    if (int rc = rp_check_args(ctx, a, true)) return rc;
+    const int64_t total_rows = a.n_items * (int64_t)a.rows_per_item;
+    rp_norm nm;
+    int rc;
+    if (rp_match_norm(a, nm) && rp_try_norm_any(ctx, a, nm, total_rows, &rc)) return rc;
+    return rp_launch_any(ctx, a, total_rows);
+}
+
+extern "C" int ktb_launch_row_program(ktb_ctx* ctx, const ktb_rowprog_args* args) {
+    if (!ctx || !args) return KTB_E_ARG;
+    const ktb_rowprog_args& a = *args;
+    if (a.n_items <= 0 || a.rows_per_item <= 0) return KTB_OK;
+    if (int rc = rp_check_args(ctx, a, false)) return rc;
     // eight vectors per thread where the row is long enough (the fold pairs the same elements whatever the
     // split; fewer, longer threads per row need fewer exchanges between warps: layer norm 8192 x 1024 takes
     // 133 us with 8 vectors per thread, 145 with 4, 162 with 2, 221 with 1)
@@ -839,7 +863,6 @@ extern "C" int ktb_launch_row_program(ktb_ctx* ctx, const ktb_rowprog_args* args
     while (T < vecs && T < 256 && a.n_items * (int64_t)a.rows_per_item / (256 / T) < 2 * (int64_t)ctx->sm_count) T *= 2;
     const int NV = vecs / T;
     const int64_t total_rows = a.n_items * (int64_t)a.rows_per_item;
-    if (total_rows >= (1ll << 31)) return ktb_fail(ctx, KTB_E_UNSUPPORTED, "row_program", "more than 2^31 rows");
     const int groups = 256 / T;
     const int64_t n_iter = (total_rows + groups - 1) / groups;
     int64_t blocks = (int64_t)ctx->sm_count * 8;
@@ -852,6 +875,8 @@ extern "C" int ktb_launch_row_program(ktb_ctx* ctx, const ktb_rowprog_args* args
             KTB_CHECK_LAUNCH(ctx, "ktb_row_norm_blocks_kernel");
             return KTB_OK;
         }
+        int rc;                                          // block counts that are no power of two, or rows too long for registers
+        if (rp_try_norm_any(ctx, a, nm, total_rows, &rc)) return rc;
     } else if (matched) {
         // four vectors per thread (the row and its squares sit in registers): two CTAs per SM
 #ifndef KTB_RP_NORM_VPT

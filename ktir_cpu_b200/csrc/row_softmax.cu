@@ -366,7 +366,7 @@ __global__ void __launch_bounds__(512) ktb_row_softmax_any_kernel(const ktb_soft
     const int t = threadIdx.x - group * T;
     const int64_t row = (int64_t)blockIdx.x * (blockDim.x / T) + group;
     if (row >= total_rows) return;                       // whole row groups: the barriers are per group
-    float* buf = rg_smem + group * (R16 ? rg_scratch(a.cols) : 32);
+    float* buf = rg_smem + group * (R16 ? rg_chunk_elems(a.cols) + rg_fold_floats(a.cols) : 32);
     const int lane = threadIdx.x & 31, warp = t >> 5, warps = T >> 5;
     const int64_t item = (uint32_t)row / (uint32_t)a.rows_per_item;
     const int64_t r = row - item * a.rows_per_item;
@@ -406,7 +406,9 @@ __global__ void __launch_bounds__(512) ktb_row_softmax_any_kernel(const ktb_soft
             for (int v = 0; v < 8; ++v) x[j][v] = ktb_round16(expf(ktb_round16(x[j][v] - mx)));
             rg_park8(buf, mis, cols, j * T + t, x[j]);
         }
-        sum = ktb_round16(rg_fold<1, MAXNUM, true>(buf, mis, cols, T, t, group) + a.sum_init);
+        const float* first = buf + mis;
+        sum = rg_fold<1, MAXNUM, true>([=](int i) { return first[i]; }, buf + rg_chunk_elems(cols), cols, T, t, group);
+        sum = ktb_round16(sum + a.sum_init);
     } else {
         float s0 = 0.f, s1 = 0.f;                        // (lanes outside the row hold -inf and add nothing)
 #pragma unroll
@@ -548,7 +550,7 @@ static int launch_softmax_any(ktb_ctx* ctx, const ktb_softmax_args& a, const rg_
         if (mn) ktb_row_softmax_any_h_kernel<NV, true><<<blocks, threads, 0, ctx->stream>>>(a, s.threads, total_rows);
         else ktb_row_softmax_any_h_kernel<NV, false><<<blocks, threads, 0, ctx->stream>>>(a, s.threads, total_rows);
     } else if constexpr (NV <= 4) {
-        const size_t smem = (r16 ? rg_scratch(a.cols) : 32) * sizeof(float) * s.groups;
+        const size_t smem = (r16 ? rg_chunk_elems(a.cols) + rg_fold_floats(a.cols) : 32) * sizeof(float) * s.groups;
         auto k = r16 ? (mn ? ktb_row_softmax_any_kernel<NV, true, true> : ktb_row_softmax_any_kernel<NV, true, false>)
                      : (mn ? ktb_row_softmax_any_kernel<NV, false, true> : ktb_row_softmax_any_kernel<NV, false, false>);
         if (smem > 48 * 1024) KTB_CUDA(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));

@@ -189,6 +189,7 @@ SYMBOLS = {
     "ktb_copy_threads": (C.c_int, []),
     "ktb_launch_ew_stream": (C.c_int, [C.c_void_p, C.POINTER(EwArgs)]),
     "ktb_launch_row_program": (C.c_int, [C.c_void_p, C.POINTER(RowProgArgs)]),
+    "ktb_launch_row_program_any": (C.c_int, [C.c_void_p, C.POINTER(RowProgArgs)]),
     "ktb_launch_row_softmax": (C.c_int, [C.c_void_p, C.POINTER(SoftmaxArgs)]),
     "ktb_launch_row_softmax_any": (C.c_int, [C.c_void_p, C.POINTER(SoftmaxArgs)]),
     "ktb_launch_rows_program": (C.c_int, [C.c_void_p, C.POINTER(RowsArgs)]),

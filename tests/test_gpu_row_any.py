@@ -56,3 +56,60 @@ def test_softmax_rows_that_start_anywhere(stride, build_lib):
     assert kinds == ["row_softmax"] and symbols == ["ktb_launch_row_softmax" + ("" if stride == 72 else "_any")]
     np.testing.assert_allclose(got["output_ptr"].astype(np.float32), want["output_ptr"].astype(np.float32), rtol=2e-3, atol=2e-6)
     np.testing.assert_array_equal(got["output_ptr"][:, cols:], 9)
+
+
+def _bits(got, want, names):
+    for k in names:
+        u = np.uint16 if want[k].dtype == np.float16 else np.uint32
+        np.testing.assert_array_equal(got[k].view(u), want[k].view(u), err_msg=k)
+
+
+# a row per warp, several warps, one CTA; one to four fold rounds; odd lengths (every row starts elsewhere), even, whole vectors
+NORM = [(24, 71, 4, 2), (24, 257, 4, 1), (64, 300, 4, 4), (40, 1000, 5, 8), (36, 1290, 3, 4), (24, 2049, 3, 1), (12, 5120, 3, 2),
+        (6, 9999, 3, 1), (4, 16383, 2, 1), (600, 264, 4, 2), (4, 512, 2, 1)]
+
+
+@pytest.mark.parametrize("rows,cols,cores,step", NORM)
+def test_rmsnorm_rows_of_any_length(rows, cols, cores, step, build_lib):
+    """The sum in the reference's fold order, every op rounded where the reference rounds: its bits."""
+    rng = np.random.default_rng(cols)
+    kw = dict(x_ptr=(rng.standard_normal((rows, cols)) * 2).astype(np.float16), w_ptr=rng.standard_normal(cols).astype(np.float16),
+              y_ptr=np.full((rows, cols), 9, np.float16), rstd_ptr=np.zeros(rows, np.float32))
+    got, want, kinds, symbols = _both(K.rmsnorm_rows(rows, cols, cores, step, weight=True), "rmsnorm_kernel", kw)
+    assert kinds == ["row_program"] and symbols == ["ktb_launch_row_program" + ("" if cols == 512 else "_any")]
+    _bits(got, want, ("y_ptr", "rstd_ptr"))
+
+
+@pytest.mark.parametrize("rows,cols,cores", [(24, 257, 4), (40, 1000, 5), (24, 2049, 3), (6, 5120, 3), (4, 16383, 2)])
+def test_layernorm_rows_of_any_length(rows, cols, cores, build_lib):
+    rng = np.random.default_rng(cols)
+    kw = dict(x_ptr=(rng.standard_normal((rows, cols)) * 3 + 1).astype(np.float16), w_ptr=rng.standard_normal(cols).astype(np.float16),
+              b_ptr=rng.standard_normal(cols).astype(np.float16), y_ptr=np.zeros((rows, cols), np.float16), mean_ptr=np.zeros(rows, np.float32))
+    got, want, kinds, _ = _both(K.layernorm_rows(rows, cols, cores), "layernorm_kernel", kw)
+    assert kinds == ["row_program"]
+    _bits(got, want, ("y_ptr", "mean_ptr"))
+
+
+@pytest.mark.parametrize("rows,block,blocks,cores", [(11, 53, 7, 3), (37, 1024, 3, 32), (9, 361, 6, 4), (12, 256, 5, 5), (5, 1500, 8, 2),
+                                                     (6, 448, 1, 3), (3, 2048, 8, 2)])
+def test_column_blocked_layernorm_of_any_length(rows, block, blocks, cores, build_lib):
+    """f16 throughout: every add of the block accumulation and of the fold rounds, in the reference's order.  (One block:
+    the block loop leaves no accumulator to recognise and Mean / Rstd / Y are statements of their own.)"""
+    rng = np.random.default_rng(block)
+    rc = (rows, block * blocks)
+    kw = dict(X=rng.standard_normal(rc).astype(np.float16), Y=np.zeros(rc, np.float16), W=rng.standard_normal(rc).astype(np.float16),
+              B=rng.standard_normal(rc).astype(np.float16), Mean=np.zeros(rows, np.float16), Rstd=np.zeros(rows, np.float16), N=rc[1],
+              eps=np.float16(1e-5), BLOCK_SIZE=block)
+    got, want, kinds, _ = _both(K.layernorm_blocked(*rc, block, cores), "_layer_norm_fwd_fused", kw)
+    assert set(kinds) == {"row_program"}
+    _bits(got, want, ("Mean", "Rstd", "Y"))
+
+
+@pytest.mark.parametrize("rows,cols,cores,step", [(24, 333, 4, 2), (12, 4000, 3, 1), (6, 16382, 3, 1)])
+def test_log_softmax_rows_of_any_length(rows, cols, cores, step, build_lib):
+    """Phases that are no normalisation: the interpreting kernel.  exp and log are the device's (f16 tolerance)."""
+    x = (np.random.default_rng(cols).standard_normal((rows, cols)) * 3).astype(np.float16)
+    got, want, kinds, symbols = _both(K.log_softmax_rows(rows, cols, cores, step), "log_softmax_kernel",
+                                      dict(x_ptr=x, y_ptr=np.zeros_like(x)))
+    assert kinds == ["row_program"] and symbols == ["ktb_launch_row_program_any"]
+    np.testing.assert_allclose(got["y_ptr"].astype(np.float32), want["y_ptr"].astype(np.float32), rtol=2e-3, atol=2e-3)
