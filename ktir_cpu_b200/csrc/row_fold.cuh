@@ -226,13 +226,31 @@ static __device__ __forceinline__ void rg_park8(float* buf, int mis, int cols, i
 }
 
 // Three levels of the reference's fold at once: of n values, level one leaves n - n / 2 — value i is x(i) (op)
-// x(i + n / 2), and an odd last one is carried along (ktir_cpu/dialects/linalg_ops.py:86-133).
-template <int OP, bool MAXNUM, bool R16, typename F>
-static __device__ __forceinline__ float rg_level3(F x, int n, int i) {
+// x(i + n / 2), and an odd last one is carried along (ktir_cpu/dialects/linalg_ops.py:86-133).  For all but the last
+// few i (none of them carried) this is eight values in a fixed pairing.
+template <typename F, typename C>
+static __device__ __forceinline__ auto rg_level3(F x, C op, int n, int i) {
     const int h0 = n >> 1, n1 = n - h0, h1 = n1 >> 1, n2 = n1 - h1, h2 = n2 >> 1;
-    auto l1 = [&](int k) { return k < h0 ? sm_comb<OP, MAXNUM, R16>(x(k), x(k + h0)) : x(k + h0); };
-    auto l2 = [&](int k) { return k < h1 ? sm_comb<OP, MAXNUM, R16>(l1(k), l1(k + h1)) : l1(k + h1); };
-    return i < h2 ? sm_comb<OP, MAXNUM, R16>(l2(i), l2(i + h2)) : l2(i + h2);
+    if (i < h2 && i + h2 < h1 && i + h2 + h1 < h0) {
+        const auto p = op(op(x(i), x(i + h0)), op(x(i + h1), x(i + h1 + h0)));
+        const auto q = op(op(x(i + h2), x(i + h2 + h0)), op(x(i + h2 + h1), x(i + h2 + h1 + h0)));
+        return op(p, q);
+    }
+    // the general form, as a loop over the eight places: those that do not exist are left out of their pair
+    auto s2 = x(0);                                      // (both are set before they are read)
+    auto s1 = s2;
+#pragma unroll 1
+    for (int e2 = 0; e2 < (i < h2 ? 2 : 1); ++e2) {
+        const int j = i < h2 ? i + e2 * h2 : i + h2;
+#pragma unroll 1
+        for (int e1 = 0; e1 < (j < h1 ? 2 : 1); ++e1) {
+            const int k = j < h1 ? j + e1 * h1 : j + h1;
+            const auto v = k < h0 ? op(x(k), x(k + h0)) : x(k + h0);
+            s1 = e1 ? op(s1, v) : v;
+        }
+        s2 = e2 ? op(s2, s1) : s1;
+    }
+    return s2;
 }
 static __host__ __device__ __forceinline__ int rg_after3(int n) {
     n -= n >> 1;
@@ -249,46 +267,79 @@ static __host__ __device__ __forceinline__ int rg_fold_floats(int cols) {
 }
 
 // Fold of value(0) .. value(cols - 1), which the T threads of the group have put where `value` finds them, in the
-// reference's order for any length; every thread gets the result, and what `value` reads is left alone.  Three levels
-// per barrier (every value is read once, an eighth of that again); the last 32 by shuffles in the first warp.
-template <int OP, bool MAXNUM, bool R16, typename F>
-static __device__ __forceinline__ float rg_fold(F value, float* tmp, int cols, int T, int t, int group) {
-    float* dst = tmp;
-    float* other = tmp + ((rg_after3(cols) + 3) & ~3);
-    float* result = tmp + rg_fold_floats(cols) - 4;
+// reference's order for any length, with `op` on values of type V; every thread gets the result, and what `value`
+// reads is left alone.  Three levels per barrier (every value is read once, an eighth of that again); the last 32 by
+// shuffles in the first warp.  `first_wide(dst)` may do the first three levels itself (whole vectors) and return true.
+template <typename V, typename F, typename C, typename W>
+static __device__ __forceinline__ V rg_fold_with(F value, C op, W first_wide, float* tmp, int cols, int T, int t, int group) {
+    V* dst = reinterpret_cast<V*>(tmp);
+    V* other = reinterpret_cast<V*>(tmp + ((rg_after3(cols) + 3) & ~3));
+    V* result = reinterpret_cast<V*>(tmp + rg_fold_floats(cols) - 4);
     rg_barrier(group, T);
     int n = cols;
-    float v = 0.f;
+    V v = V();
     if (n > 256) {
         const int m = rg_after3(n);
-        for (int i = t; i < m; i += T) dst[i] = rg_level3<OP, MAXNUM, R16>(value, n, i);
+        if (!first_wide(dst))
+            for (int i = t; i < m; i += T) dst[i] = rg_level3(value, op, n, i);
         n = m;
         rg_barrier(group, T);
         while (n > 256) {
             const int k = rg_after3(n);
-            const float* src = dst;
-            for (int i = t; i < k; i += T) other[i] = rg_level3<OP, MAXNUM, R16>([&](int q) { return src[q]; }, n, i);
+            const V* src = dst;
+            for (int i = t; i < k; i += T) other[i] = rg_level3([&](int q) { return src[q]; }, op, n, i);
             rg_barrier(group, T);
-            float* o = dst;
+            V* o = dst;
             dst = other;
             other = o;
             n = k;
         }
-        if (t < 32 && t < rg_after3(n)) v = rg_level3<OP, MAXNUM, R16>([&](int q) { return dst[q]; }, n, t);
+        if (t < 32 && t < rg_after3(n)) v = rg_level3([&](int q) { return dst[q]; }, op, n, t);
     } else if (t < 32 && t < rg_after3(n)) {
-        v = rg_level3<OP, MAXNUM, R16>(value, n, t);
+        v = rg_level3(value, op, n, t);
     }
     if (t < 32) {
         for (n = rg_after3(n); n > 1;) {
             const int h = n >> 1;
-            const float o = __shfl_down_sync(0xffffffffu, v, h);
-            v = t < h ? sm_comb<OP, MAXNUM, R16>(v, o) : o;
+            const V o = __shfl_down_sync(0xffffffffu, v, h);
+            v = t < h ? op(v, o) : o;
             n -= h;
         }
         if (t == 0) *result = v;
     }
     rg_barrier(group, T);
     return *result;
+}
+template <int OP, bool MAXNUM, bool R16, typename F>
+static __device__ __forceinline__ float rg_fold(F value, float* tmp, int cols, int T, int t, int group) {
+    return rg_fold_with<float>(value, [](float a, float b) { return sm_comb<OP, MAXNUM, R16>(a, b); },
+                               [](float*) { return false; }, tmp, cols, T, t, group);
+}
+
+// Two f32 values in one 64-bit register: fma / add / mul on such a pair are ONE instruction here, each half rounded like
+// the scalar op.
+static __device__ __forceinline__ uint64_t sm_pack2(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+static __device__ __forceinline__ void sm_unpack2(uint64_t v, float& lo, float& hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+static __device__ __forceinline__ uint64_t sm_fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+static __device__ __forceinline__ uint64_t sm_add2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+static __device__ __forceinline__ uint64_t sm_mul2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
 }
 
 // The same fold of a sum whose every add rounds to f16, on packed halves: an f16 add of two f16 values is

@@ -11,6 +11,7 @@
 // back (linalg_ops.py:349-465) and the elementwise ops around them, with the same rounding points
 // (f16 tiles round after every op, f32 tiles do not).
 #include "row_fold.cuh"
+#include "tc_common.cuh"
 #include "vm.cuh"
 
 template <int NV>
@@ -381,7 +382,7 @@ template <int NV, int MODE, bool PER_ROW>
 #ifndef KTB_RP_NORM_OCC
 #define KTB_RP_NORM_OCC 3
 #endif
-__global__ void __launch_bounds__(256, NV >= 8 ? 1 : NV >= 4 ? KTB_RP_NORM_OCC : NV >= 2 ? 3 : 4)
+__global__ void __launch_bounds__(256, NV >= 4 ? KTB_RP_NORM_OCC : NV >= 2 ? 3 : 4)
 ktb_row_norm_kernel(const __grid_constant__ ktb_rowprog_args a, const rp_norm m, int T, int64_t total_rows) {
     __shared__ float xchg[256 * 8];
     __shared__ float bcast[8];
@@ -870,15 +871,23 @@ extern "C" int ktb_launch_row_program(ktb_ctx* ctx, const ktb_rowprog_args* args
 #ifndef KTB_RP_NO_NORM
     rp_norm nm;
     const bool matched = rp_match_norm(a, nm);
+    // Rows of more than 512 elements, and few rows of any length, go to the kernel that parks the row in shared memory:
+    // layer norm f16[2048, 8192] 28.9 us against 69.5 in registers, blocked f16[4096, 8 x 1024] 59.2 against 82.1,
+    // [8192, 1024] 20.6 against 31.0, [256, 256] 6.2 against 9.8.  Many short rows stay in registers, several to a
+    // warp: [16384, 512] 30.3 against 34.2, [32768, 128] 20.2 against 41.0.
+    int rc_any;
+    if (matched && ((int64_t)(nm.blocked ? a.n_blocks : 1) * a.cols > 512 || total_rows <= 2048) &&
+        rp_try_norm_any(ctx, a, nm, total_rows, &rc_any))
+        return rc_any;
     if (matched && (nm.blocked || nm.r16)) {
         if (rp_try_norm_blocks(ctx, a, nm, total_rows)) {
             KTB_CHECK_LAUNCH(ctx, "ktb_row_norm_blocks_kernel");
             return KTB_OK;
         }
-        int rc;                                          // block counts that are no power of two, or rows too long for registers
-        if (rp_try_norm_any(ctx, a, nm, total_rows, &rc)) return rc;
+        // block counts that are no power of two
+        if (rp_try_norm_any(ctx, a, nm, total_rows, &rc_any)) return rc_any;
     } else if (matched) {
-        // four vectors per thread (the row and its squares sit in registers): two CTAs per SM
+        // four vectors per thread (the row and its squares sit in registers): two CTAs per SM; rows of 512 at most
 #ifndef KTB_RP_NORM_VPT
 #define KTB_RP_NORM_VPT 4
 #endif
@@ -892,7 +901,6 @@ extern "C" int ktb_launch_row_program(ktb_ctx* ctx, const ktb_rowprog_args* args
             case 1: rp_launch_norm<1>(ctx, a, nm, bn, Tn, total_rows); break;
             case 2: rp_launch_norm<2>(ctx, a, nm, bn, Tn, total_rows); break;
             case 4: rp_launch_norm<4>(ctx, a, nm, bn, Tn, total_rows); break;
-            case 8: rp_launch_norm<8>(ctx, a, nm, bn, Tn, total_rows); break;
             default: return ktb_fail(ctx, KTB_E_UNSUPPORTED, "row_program", "unsupported row width");
         }
         KTB_CHECK_LAUNCH(ctx, "ktb_row_norm_kernel");

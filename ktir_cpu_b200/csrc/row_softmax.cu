@@ -131,32 +131,6 @@ static __device__ __forceinline__ void sm_row_exp(const uint4& raw, float mxs, f
     }
 }
 
-// Two f32 values in one 64-bit register: Blackwell issues fma / add / mul on such a pair as ONE instruction,
-// which takes a third off the instruction count of a row (the kernel is issue-bound next to HBM-bound).
-static __device__ __forceinline__ uint64_t sm_pack2(float lo, float hi) {
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-static __device__ __forceinline__ void sm_unpack2(uint64_t v, float& lo, float& hi) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-static __device__ __forceinline__ uint64_t sm_fma2(uint64_t a, uint64_t b, uint64_t c) {
-    uint64_t r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-static __device__ __forceinline__ uint64_t sm_add2(uint64_t a, uint64_t b) {
-    uint64_t r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-static __device__ __forceinline__ uint64_t sm_mul2(uint64_t a, uint64_t b) {
-    uint64_t r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-
 // exp of the 8 values of one vector, parked in place as f16: p * 2^15 = 2^(x log2e - (m log2e - 15)), the scale
 // folded into the exponent (0 < p <= 1, so p * 2^15 keeps 11 significant bits down to p = 2^-29); the two
 // accumulators collect the same scaled values in f32.

@@ -207,16 +207,17 @@ def _signature(n: Node, loads: List[Node], fixed: Dict[int, int]):
     return ("?", id(n))
 
 
-def _block_chain(src: Node):
+def _block_chain(src: Node, least: int):
     """``src = (((init + t_0) + t_1) + ... + t_{B-1})``, the accumulator a column-blocked kernel carries
-    through its loop over the blocks of a row: (init value, [t_0 ...], adds round to f16) or None."""
+    through its loop over the blocks of a row: (init value, [t_0 ...], adds round to f16) or None if there are
+    fewer than ``least`` terms."""
     terms = []
     n = _canon(src)
     dtype = n.dtype
     while n.kind == "ew" and n.attrs.get("op") == "arith.addf" and len(n.args) == 2 and n.dtype == dtype:
         terms.append(n.args[1])
         n = _canon(n.args[0])
-    if n.kind != "const" or n.attrs.get("list") is not None or len(terms) < 2:
+    if n.kind != "const" or n.attrs.get("list") is not None or len(terms) < least:
         return None
     terms.reverse()
     return float(n.attrs["value"]), terms, dtype == "f16"
@@ -249,7 +250,7 @@ class RowProgramStatement(Statement):
         cols, full = int(src_shape[-1]), _prod(src_shape)
         if cols > 16384:
             raise Unsupported(f"row program over rows of {cols} elements (16384 at most)")
-        plain = cols >= 8 and not cols & (cols - 1)          # 2^n columns; cleared below where a row starts off a boundary
+        aligned = True                                       # cleared below where a row starts off a boundary
         rows_total = full // cols
         per_row = _prod(tgt.shape) == rows_total and rows_total != full
         if not per_row and _prod(tgt.shape) != full:
@@ -260,6 +261,8 @@ class RowProgramStatement(Statement):
         axes = tuple(store.axes)
         sel_all, cores_all = _points(store)
         chains = {}
+        # (a single block is a chain of one term, init + x: only inside a loop of one trip that stores the row)
+        least = 1 if not per_row and len(axes) >= 2 and axes[-1] == 1 else 2
 
         def find_chains(n: Node, seen):
             n = strip_views(n)
@@ -267,7 +270,7 @@ class RowProgramStatement(Statement):
                 return
             seen.add(id(n))
             if n.kind == "reduce":
-                c = _block_chain(n.args[0])
+                c = _block_chain(n.args[0], least)
                 if c is not None:
                     chains[id(n)] = c
             for a_ in n.args:
@@ -517,7 +520,7 @@ class RowProgramStatement(Statement):
             if o.blk_stride < 0:
                 raise Unsupported("row program over column blocks that run backwards")
             if (offs % 8).any() or (g.rows > 1 and g.row_stride % 8) or o.blk_stride % 8:
-                plain = False
+                aligned = False
         bpe = bytes_per_elem(tgt.view.dtype)
         a.dtype[n_in] = R.DTYPE_CODE[tgt.view.dtype]
         if per_row:
@@ -537,25 +540,26 @@ class RowProgramStatement(Statement):
                                   (n_blocks - 1) * max(out_step, 0) + go.cols, tgt.view.dtype, "Scatter to")
             footprint(offs, go, out_step if absorb else 0, bpe, True)
             a.row_stride[n_in] = 8 if go.rows == 1 else go.row_stride
-            if out_step < 0 or (absorb and out_step == 0):
+            if out_step < 0 or (absorb and out_step == 0 and n_blocks > 1):
                 raise Unsupported("row program whose output blocks do not advance")
             if (offs % 8).any() or (go.rows > 1 and go.row_stride % 8) or out_step % 8:
-                plain = False
+                aligned = False
         a.n_items, a.rows_per_item, a.cols = table.shape[0], g0.rows, cols
-        # Aligned rows of 2^n elements have kernels of their own (the row in registers, the fold by shuffles), which
-        # are faster there: rms norm f16[32768, 128] 14.4 us against 39.6, [2048, 8192] 45.1 against 48.9, blocked
-        # layer norm f16[4096, 8 x 1024] 81.6 against 196; every other row goes to the kernels for any length.
-        # Normalisations with two reductions on rows of less than 256 such elements stay step by step although the
-        # kernel could take them: they are what the tests check that path with.
-        if not plain and cols * n_blocks < 256 and n_red > 1:
-            raise Unsupported(f"row program with {n_red} reductions over rows of {cols * n_blocks} elements")
+        # Aligned rows of 2^n elements: the launcher that also has kernels with the row in registers, for many short rows
+        # (rms norm f16[32768, 128] 14.4 us against 28.8); every other row only has the kernels for any length.
+        # Layer norms (two reductions, the mean beside them) on rows of less than 256 such elements stay step by step
+        # although the kernel could take them: they are what the tests check that path with.
+        plain = aligned and cols >= 8 and not cols & (cols - 1)
+        if not plain and cols * n_blocks < 256 and (n_red > 1 or per_row):
+            raise Unsupported(f"row program over rows of {cols * n_blocks} elements")
+        a.aligned = int(aligned)
         self.symbol = "ktb_launch_row_program" if plain else "ktb_launch_row_program_any"
         self.table = table
         self._sel, self._n_lead, self._dev, self.rounds = sel, n_lead, dev, None
         self.stores = [store]
         self._side_ctx = None if per_row or n_lead != 1 else dict(
             red_index=red_index, n_red=n_red, rows_total=rows_total, axes=axes, cores=cores, rows=g0.rows,
-            div=n_blocks if absorb else 1, arena=arena, stmt_id=stmt_id)
+            div=n_blocks if absorb else 1, absorb=absorb, arena=arena, stmt_id=stmt_id)
         self.dev_table = dev.upload(table)
         a.dev_item_offsets = self.dev_table
         self.device_arrays = [self.dev_table]
@@ -579,7 +583,7 @@ class RowProgramStatement(Statement):
         # the same iteration points: the side store sits at this statement's loop depth, or one level above the
         # loop over column blocks this statement has absorbed
         s_axes = tuple(side.axes)
-        if s_axes != (axes if c["div"] == 1 else axes[:-1]):
+        if s_axes != (axes[:-1] if c["absorb"] else axes):
             return False
         s_sel, s_cores = _points(side)
         if len(s_sel) != len(self._sel) or (s_sel != self._sel // c["div"]).any() or (s_cores != c["cores"]).any():

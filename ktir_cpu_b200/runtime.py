@@ -71,7 +71,7 @@ class RowProgArgs(C.Structure):
                 ("row_stride", C.c_int64 * (VM_MAX_IN + 1)), ("dtype", C.c_int32 * (VM_MAX_IN + 1)),
                 ("blk_stride", C.c_int64 * (VM_MAX_IN + 1)), ("n_blocks", C.c_int32), ("n_side", C.c_int32),
                 ("red", RpPhase * RP_MAX_RED), ("scal", RpScalar * RP_MAX_SCAL), ("out", RpPhase),
-                ("side", RpSide * RP_MAX_SIDE)]
+                ("side", RpSide * RP_MAX_SIDE), ("aligned", C.c_int32), ("reserved", C.c_int32)]
 
 
 class SoftmaxArgs(C.Structure):
