@@ -146,6 +146,11 @@ enum {
     KTB_VM_MAX, KTB_VM_MAXNUM, KTB_VM_MIN, KTB_VM_MINNUM, KTB_VM_NEG, KTB_VM_ABS,
     KTB_VM_EXP, KTB_VM_LOG, KTB_VM_LOG2, KTB_VM_SQRT, KTB_VM_RSQRT, KTB_VM_TANH,
     KTB_VM_SIN, KTB_VM_COS, KTB_VM_FMA, KTB_VM_NOPS,
+    /* programs of ktb_launch_ew_multi only.  CSEL: select(cmp(a, b), c, f), imm = 8 * (KTB_CMP_* set) + f;
+       RSQRT_STEPS: 1 / sqrt(a), both steps rounded under KTB_VM_ROUND16 (ktir_cpu/ops/math_ops.py:38-41);
+       ERF: the polynomial the reference evaluates op by op in the tile's dtype (math_ops.py:99-111), f16 steps under
+       KTB_VM_ROUND16 */
+    KTB_VM_CSEL = KTB_VM_NOPS, KTB_VM_RSQRT_STEPS, KTB_VM_ERF, KTB_VM_ALL_OPS,
     KTB_VM_ROUND16 = 0x100,
     /* row-value programs of ktb_launch_row_program only (row scalars, per-row and side results): operand a / b of
        the op is `imm` instead of a register, which saves the KTB_VM_CONST op in front of it */
@@ -187,6 +192,24 @@ typedef struct {
     ktb_vm_program program;
 } ktb_ew_args;
 int ktb_launch_ew_stream(ktb_ctx* ctx, const ktb_ew_args* args);
+/* Several stores over the same items and tile shape in one launch: the input tiles are read once, every output has a
+ * program of its own over them.  No output may share bytes with an input or another output, except a single output
+ * with an input tile that is the same tile.  item_offsets: [n_items][n_in + n_out]. */
+#define KTB_EW_MAX_OUT 8
+/* A comparison is the set of outcomes it holds for (arith.cmpf `ule`: LT | EQ | UNORDERED). */
+enum { KTB_CMP_LT = 1, KTB_CMP_EQ = 2, KTB_CMP_GT = 4, KTB_CMP_UNORDERED = 8 };
+typedef struct {
+    void* arena;
+    const int64_t* dev_item_offsets;
+    int64_t n_items;
+    int32_t rows, cols, n_in, n_out;
+    int64_t row_stride[KTB_VM_MAX_IN + KTB_EW_MAX_OUT];   /* elements; inputs, then outputs */
+    int32_t dtype[KTB_VM_MAX_IN + KTB_EW_MAX_OUT];        /* KTB_F16 / KTB_F32 */
+    int32_t vector_ok;                                    /* as in ktb_ew_args */
+    int32_t reserved;
+    ktb_vm_program program[KTB_EW_MAX_OUT];
+} ktb_ew_multi_args;
+int ktb_launch_ew_multi(ktb_ctx* ctx, const ktb_ew_multi_args* args);
 
 /* ---- fused row softmax --------------------------------------------------------
  * load -> [extf] -> reduce(max) -> sub -> exp -> reduce(add) -> div -> [truncf]

@@ -22,6 +22,7 @@ COMMON = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-I", INCLUDE
 # Element-wise kernels must not contract a*b+c: each KTIR op rounds on its own.
 PER_FILE = {
     "ew_stream.cu": ["--fmad=false"],
+    "ew_multi.cu": ["--fmad=false"],
     "row_softmax.cu": ["--fmad=false"],
     "row_program.cu": ["--fmad=false"],
     "scatter_rows.cu": ["--fmad=false"],

@@ -89,9 +89,9 @@ def _copy_args(args):
     return type(args).from_buffer_copy(args)
 
 
-def _split_item_table(stmt, table: np.ndarray, geoms, bpes, launch_fn, piece_bytes: int):
-    """Split a statement whose work is rows of an item table ``[n_items][operands]`` (the last
-    operand is the output) into contiguous item ranges."""
+def _split_item_table(stmt, table: np.ndarray, geoms, bpes, launch_fn, piece_bytes: int, n_out: int = 1):
+    """Split a statement whose work is rows of an item table ``[n_items][operands]`` (the last ``n_out``
+    operands are outputs) into contiguous item ranges."""
     from .pipeline import Chunk, chunk_count, tile_regions
     n_items, n_op = table.shape
     total = sum(n_items * g[0] * g[2] * b for g, b in zip(geoms, bpes))
@@ -108,7 +108,8 @@ def _split_item_table(stmt, table: np.ndarray, geoms, bpes, launch_fn, piece_byt
             if r is None:
                 return None
             regs.append(r)
-        chunks.append(Chunk(launch_fn(int(a), int(b)), [x for r in regs[:-1] for x in r], list(regs[-1])))
+        chunks.append(Chunk(launch_fn(int(a), int(b)), [x for r in regs[:-n_out] for x in r],
+                            [x for r in regs[-n_out:] for x in r]))
     return chunks
 
 
@@ -190,7 +191,9 @@ def strip_views(n: Node) -> Node:
 class ProgramBuilder:
     """Compiles an elementwise DAG over same-shaped tiles into a register program."""
 
-    def __init__(self, leaf_kinds=("load",)):
+    def __init__(self, leaf_kinds=("load",), extended: bool = False):
+        """``extended``: the ops that only ``ktb_launch_ew_multi`` has may be used (``self.used_extra`` says so)."""
+        self.extended, self.used_extra = extended, False
         self.inputs: List[Node] = []
         self.ops: List[Tuple[int, int, int, int, int, float]] = []
         self.reg_of: Dict[int, int] = {}
@@ -225,9 +228,13 @@ class ProgramBuilder:
     def emit(self, code: str, dst: int, a=0, b=0, c=0, imm=0.0, r16=False):
         if len(self.ops) >= R.VM_MAX_OPS:
             raise Unsupported("elementwise expression longer than 12 ops")
-        self.ops.append((R.VM[code] | (R.VM_ROUND16 if r16 else 0), dst, a, b, c, float(imm)))
+        if code in R.VM_EXTRA:
+            self.used_extra = True
+        self.ops.append(((R.VM_EXTRA[code] if code in R.VM_EXTRA else R.VM[code]) | (R.VM_ROUND16 if r16 else 0), dst, a, b, c, float(imm)))
 
-    def build(self, root: Node, full_shape: Tuple[int, ...]) -> R.VmProgram:
+    def build(self, root: Node, full_shape: Tuple[int, ...], place=None) -> R.VmProgram:
+        """``place`` = (register of an input node, registers taken by inputs): where a program that shares its inputs
+        with others finds them; otherwise they come in the order they are met."""
         self.collect_inputs(root)
         if not self.inputs:
             raise Unsupported("store of a tile that reads no memory")
@@ -235,21 +242,52 @@ class ProgramBuilder:
             raise Unsupported(f"elementwise statement with more than {R.VM_MAX_IN} input tiles")
         self.full_elems = int(np.prod(full_shape)) if full_shape else 1
         for i, n in enumerate(self.inputs):
-            self.reg_of[id(n)] = i
-        self.next_reg = len(self.inputs)
+            self.reg_of[id(n)] = i if place is None else place[0](n)
+        n_in = self.next_reg = len(self.inputs) if place is None else place[1]
         res = self.visit(root)
+        # a final rounding of the last op's own result is that op's rounding
+        if self.extended and len(self.ops) >= 2:
+            code, dst, a = self.ops[-1][:3]
+            prev = self.ops[-2]
+            if code == (R.VM["MOV"] | R.VM_ROUND16) and dst == res and a == prev[1] and not prev[0] & R.VM_ROUND16 and \
+                    prev[0] not in R.VM_EXTRA.values():
+                self.ops[-2:] = [(prev[0] | R.VM_ROUND16, dst) + prev[2:]]
         p = R.VmProgram()
-        p.n_in, p.n_ops, p.result_reg = len(self.inputs), len(self.ops), res
+        p.n_in, p.n_ops, p.result_reg = n_in, len(self.ops), res
         for i, (code, dst, a, b, c, imm) in enumerate(self.ops):
             p.ops[i] = R.VmOp(code, dst, a, b, c, imm)
         return p
+
+    def check_shape(self, a: Node):
+        sa = strip_views(a)
+        if sa.kind not in ("const",) and not (sa.kind == "bcast" and strip_views(sa.args[0]).kind == "const"):
+            if int(np.prod(sa.shape)) != self.full_elems:
+                raise Unsupported("broadcasting between tiles of different shape in an elementwise statement")
 
     def visit(self, n: Node) -> int:
         n = strip_views(n)
         if id(n) in self.reg_of:
             return self.reg_of[id(n)]
         r16 = n.dtype == "f16"
-        if n.kind == "const":
+        if self.extended and n.kind == "ew" and n.dtype in F_DT and "steps_of" in n.attrs:
+            code, x = n.attrs["steps_of"]
+            self.check_shape(x)
+            src = self.visit(x)
+            r = self.alloc()
+            self.emit(code, r, src, r16=r16)
+        elif self.extended and n.kind == "ew" and n.dtype in F_DT and n.attrs["op"] == "arith.select" and \
+                strip_views(n.args[0]).kind == "ew" and strip_views(n.args[0]).attrs["op"] == "arith.cmpf" and \
+                strip_views(n.args[0]).attrs["pred"] in R.CMP:
+            cond = strip_views(n.args[0])
+            args = list(cond.args) + list(n.args[1:])
+            if any(x.dtype not in F_DT for x in args):
+                raise Unsupported("select on other than float tiles in an elementwise statement")
+            for x in args:
+                self.check_shape(x)
+            ra, rb, rt, rf = [self.visit(x) for x in args]
+            r = self.alloc()
+            self.emit("CSEL", r, ra, rb, rt, imm=8 * R.CMP[cond.attrs["pred"]] + rf, r16=r16)
+        elif n.kind == "const":
             if n.attrs.get("list") is not None:
                 raise Unsupported("dense list constant in an elementwise statement")
             v = n.attrs["value"]
@@ -269,11 +307,7 @@ class ProgramBuilder:
         elif n.kind == "ew":
             op = n.attrs["op"]
             for a in n.args:
-                sa = strip_views(a)
-                if sa.kind not in ("const",) and not (sa.kind == "bcast" and strip_views(sa.args[0]).kind == "const"):
-                    if int(np.prod(sa.shape)) != self.full_elems:
-                        raise Unsupported("broadcasting between tiles of different shape in an "
-                                          "elementwise statement")
+                self.check_shape(a)
             if n.dtype not in F_DT:
                 raise Unsupported(f"{op} producing {n.dtype} in an elementwise statement")
             regs = [self.visit(a) for a in n.args]
@@ -293,12 +327,13 @@ class ProgramBuilder:
 
 
 class EwStatement(Statement):
+    """Elementwise ops between loads and a store; neighbouring stores over the same tiles join it (``try_merge``)."""
     kind = "ew_stream"
 
     def __init__(self, dev: R.Device, store: Store, arena: ArenaMap, stmt_id: int):
         tgt: Access = store.target
-        pb = ProgramBuilder()
-        self.program = pb.build(store.value, tgt.shape)
+        pb = ProgramBuilder(extended=True)
+        program = pb.build(store.value, tgt.shape)
         operands: List[Access] = [n.attrs["access"] for n in pb.inputs] + [tgt]
         n_elems = int(np.prod(tgt.shape)) if tgt.shape else 1
         for acc in operands[:-1]:
@@ -312,51 +347,125 @@ class EwStatement(Statement):
         sel, cores = _points(store)
         self.n_points = len(sel)
         n_lead = len(g_out.lead)
-        table = np.empty((len(sel) * n_lead, len(operands)), np.int64)
-        self.fps: List[Footprint] = []
+        self._sel, self._n_lead, self._dev, self.rounds = sel, n_lead, dev, None
+        self._cores, self._rows, self._cols, self._id = cores, g_out.rows, g_out.cols, stmt_id
+        # operand columns of the item table: (offsets, row stride, dtype, footprint)
+        self._cols_of: List[tuple] = []
         for k, (acc, g) in enumerate(zip(operands, geoms)):
             offs = _access_offsets(acc, store, sel)
             full = (offs[:, None] + g.lead[None, :]).reshape(-1)
-            table[:, k] = full
             if len(full):
                 span = (g.rows - 1) * g.row_stride + g.cols
                 arena.check_range(int(full.min()), int(full.max()) + span, acc.view.dtype,
                                   "Read from" if k < len(operands) - 1 else "Scatter to")
             bpe = bytes_per_elem(acc.view.dtype)
             rstart = (full[:, None] + np.arange(g.rows, dtype=np.int64)[None, :] * g.row_stride).reshape(-1) * bpe
-            pts = np.repeat(sel, n_lead * g.rows)
-            self.fps.append(Footprint(rstart, rstart + g.cols * bpe, pts, np.repeat(cores, n_lead * g.rows),
-                                      k == len(operands) - 1, stmt_id))
-        self.table = table
-        self._sel, self._n_lead, self._dev, self.rounds = sel, n_lead, dev, None
-        self.args = R.EwArgs()
-        a = self.args
-        a.n_items = table.shape[0]
-        a.rows, a.cols = g_out.rows, g_out.cols
-        vec = (g_out.cols % 8 == 0) and bool((table % 8 == 0).all())
-        for k, (acc, g) in enumerate(zip(operands, geoms)):
-            a.row_stride[k] = g.row_stride
-            a.dtype[k] = R.DTYPE_CODE[acc.view.dtype]
-            vec = vec and (g.row_stride % 8 == 0 or g.rows == 1)
+            fp = Footprint(rstart, rstart + g.cols * bpe, np.repeat(sel, n_lead * g.rows), np.repeat(cores, n_lead * g.rows),
+                           k == len(operands) - 1, stmt_id)
+            self._cols_of.append((full, g.row_stride, acc.view.dtype, fp))
+        self._n_in = len(pb.inputs)
+        self._nodes = {id(n): k for k, n in enumerate(pb.inputs)}          # input node -> operand column
+        self._stores = [store]
+        self._programs, self._extra = [program], pb.used_extra
+        self.dev_table = None
+        self._bind()
+
+    def _bind(self):
+        """Launch arguments and the item table of what the statement holds now."""
+        n_in, n_op = self._n_in, len(self._cols_of)
+        self.table = table = np.ascontiguousarray(np.stack([c[0] for c in self._cols_of], axis=1))
+        vec = (self._cols % 8 == 0) and bool((table % 8 == 0).all()) and \
+            all(c[1] % 8 == 0 or self._rows == 1 for c in self._cols_of)
+        # One add / sub / mul / div / max / min / copy has a kernel compiled for it, which runs at the copy rate (f32
+        # add of 2^24 elements 33.4 us for 201 MB); all else goes to the kernel that decodes its ops (exp of as many
+        # 34.9 us for 134 MB).
+        p = self.program = self._programs[0]
+        special = p.n_ops == 0 and p.result_reg == 0 and n_in == 1
+        if p.n_ops == 1:
+            op = p.ops[0]
+            code = R.VM_OPS[op.opcode & 0xff] if (op.opcode & 0xff) < len(R.VM_OPS) else ""
+            special = op.a == 0 and op.dst == p.result_reg and \
+                (code == "MOV" or (n_in == 2 and op.b == 1 and code in ("ADD", "SUB", "MUL", "DIV", "MAX", "MIN")))
+        self._multi = len(self._programs) > 1 or self._extra or not special
+        self.symbol = "ktb_launch_ew_multi" if self._multi else "ktb_launch_ew_stream"
+        self.args = a = R.EwMultiArgs() if self._multi else R.EwArgs()
+        a.n_items, a.rows, a.cols = table.shape[0], self._rows, self._cols
+        for k, (_, stride, dt, _) in enumerate(self._cols_of):
+            a.row_stride[k], a.dtype[k] = stride, R.DTYPE_CODE[dt]
         a.vector_ok = 1 if vec else 0
-        a.program = self.program
-        self.dev_table = dev.upload(table)
+        if self._multi:
+            a.n_in, a.n_out = n_in, n_op - n_in
+            for k, prog in enumerate(self._programs):
+                a.program[k] = prog
+        else:
+            a.program = p
+        if self.dev_table is not None:
+            self._dev.free(self.dev_table)
+        self.dev_table = self._dev.upload(table)
         a.dev_item_offsets = self.dev_table
         self.device_arrays = [self.dev_table]
-        self.elems = int(table.shape[0]) * g_out.rows * g_out.cols
-        self._bytes = sum(self.elems * bytes_per_elem(acc.view.dtype) for acc in operands)
+        self.fps = [c[3] for c in self._cols_of]
+        self.elems = int(table.shape[0]) * self._rows * self._cols
+        self._bytes = sum(self.elems * bytes_per_elem(c[2]) for c in self._cols_of)
+
+    def try_merge(self, other: "EwStatement") -> bool:
+        """Take over the statement behind this one: the same iteration points and tile shape, at most four input tiles
+        together, and all bytes written apart from everything else the two touch (so that reading all inputs first and
+        storing tile after tile, chunk by chunk, is what running one after the other gives).  The inputs are then read
+        once.  False (and nothing changed) if it does not fit."""
+        mine = (self._n_lead, self._rows, self._cols, tuple(self._stores[0].axes))
+        if mine != (other._n_lead, other._rows, other._cols, tuple(other._stores[0].axes)) or \
+                len(self._programs) + len(other._programs) > R.EW_MAX_OUT or len(self._sel) != len(other._sel) or \
+                not len(self._sel) or (self._sel != other._sel).any() or (self._cores != other._cores).any():
+            return False
+
+        def key(c):
+            return (c[0].tobytes(), c[1], c[2])
+        n0, n1 = self._n_in, other._n_in
+        ins = list(self._cols_of[:n0])
+        where = {key(c): k for k, c in enumerate(ins)}
+        for c in other._cols_of[:n1]:
+            if key(c) not in where:
+                where[key(c)] = len(ins)
+                ins.append(c)
+        if len(ins) > R.VM_MAX_IN:
+            return False
+        outs = self._cols_of[n0:] + other._cols_of[n1:]
+        for k, w in enumerate(outs):
+            for c in ins + outs[k + 1:]:
+                if _runs_overlap(w[3].starts, w[3].ends, c[3].starts, c[3].ends):
+                    return False
+        nodes = dict(self._nodes)
+        for i, k in other._nodes.items():
+            nodes[i] = where[key(other._cols_of[k])]
+        programs, extra = [], False
+        try:
+            for st in self._stores + other._stores:
+                pb = ProgramBuilder(extended=True)
+                programs.append(pb.build(st.value, st.target.shape, place=(lambda n: nodes[id(n)], len(ins))))
+                extra = extra or pb.used_extra
+        except Unsupported:                       # (more inputs leave fewer registers)
+            return False
+        for c in other._cols_of:
+            c[3].stmt = self._id
+        self._dev.free(other.dev_table)
+        self._n_in, self._nodes, self._programs, self._extra = len(ins), nodes, programs, extra
+        self._cols_of, self._stores = ins + outs, self._stores + other._stores
+        self._bind()
+        return True
 
     def launch(self, dev, arena_ptr):
         self.args.arena = arena_ptr
+        go = getattr(dev.lib, self.symbol)
         if self.rounds:                       # several points store to the same bytes: in sequential order
             n_op = self.table.shape[1]
             for lo, hi in self.rounds:
                 sub = _copy_args(self.args)
                 sub.dev_item_offsets = self.dev_table + lo * n_op * 8
                 sub.n_items = hi - lo
-                dev.check(dev.lib.ktb_launch_ew_stream(dev.h, C.byref(sub)))
+                dev.check(go(dev.h, C.byref(sub)))
             return
-        dev.check(dev.lib.ktb_launch_ew_stream(dev.h, C.byref(self.args)))
+        dev.check(go(dev.h, C.byref(self.args)))
 
     def order_points(self, rounds: Dict[int, int]):
         _order_item_table(self, self._sel, self._n_lead, rounds, self._dev)
@@ -372,14 +481,25 @@ class EwStatement(Statement):
             sub = _copy_args(a)
             sub.dev_item_offsets = self.dev_table + lo * n_op * 8
             sub.n_items = hi - lo
-            return ("ktb_launch_ew_stream", sub)
-        return _split_item_table(self, self.table, geoms, bpes, part, piece_bytes)
+            return (self.symbol, sub)
+        return _split_item_table(self, self.table, geoms, bpes, part, piece_bytes, n_out=n_op - self._n_in)
 
     def footprints(self):
         return self.fps
 
     def bytes_moved(self):
         return self._bytes
+
+
+def _runs_overlap(s0, e0, s1, e1) -> bool:
+    """True if some run [s0, e0) meets some run [s1, e1)."""
+    if not len(s0) or not len(s1) or s0.min() >= e1.max() or s1.min() >= e0.max():
+        return False
+    order = np.argsort(s1, kind="stable")
+    s1, e1 = s1[order], np.maximum.accumulate(e1[order])
+    k = np.searchsorted(s1, e0, side="left") - 1          # last run of the second set that starts before each e0
+    ok = k >= 0
+    return bool((e1[k[ok]] > s0[ok]).any())
 
 
 # ---------------------------------------------------------------------------
@@ -746,7 +866,7 @@ def lower_core_groups(dev: R.Device, trace_cores, n_cores: int, arena: ArenaMap,
                 break
             except CoreOrderHazard as plain:
                 try:
-                    lower(probe, trace_cores(lo, lo + size, True), arena, fused=fused)
+                    lower(probe, trace_cores(lo, lo + size, True), arena, fused=fused, merge=False)
                     unroll = True
                     break
                 except Unsupported as unrolled:
@@ -758,7 +878,7 @@ def lower_core_groups(dev: R.Device, trace_cores, n_cores: int, arena: ArenaMap,
     plan = Plan()
     try:
         for lo, hi, unroll in groups:
-            part = lower(dev, trace_cores(lo, hi, unroll), arena, fused=fused)
+            part = lower(dev, trace_cores(lo, hi, unroll), arena, fused=fused, merge=not unroll)
             plan.statements.extend(part.statements)
             plan.written |= part.written
     except Exception:
@@ -799,10 +919,11 @@ def _fused_statement(dev, st: Store, arena: ArenaMap, sid: int, row_shard):
 FUSE_ROW_RESULTS = True
 
 
-def lower(dev: R.Device, stores: List[Store], arena: ArenaMap, row_shard=None, fused: bool = True) -> Plan:
+def lower(dev: R.Device, stores: List[Store], arena: ArenaMap, row_shard=None, fused: bool = True, merge: bool = True) -> Plan:
     """``row_shard = (rank, world)``: ordered scatters apply only the destination rows this rank owns.
     ``fused=False`` skips the fused kernels and runs every direct store step by step (the op-by-op
-    form of the reference, ktir_cpu/interpreter.py:196-281) — a cross-check for the fused paths."""
+    form of the reference, ktir_cpu/interpreter.py:196-281) — a cross-check for the fused paths.
+    ``merge=False`` keeps every elementwise store a launch of its own (iterations that run one by one)."""
     from .order import program_order
     stores = [stores[k] for k in program_order(stores, arena)]
     plan = Plan()
@@ -829,6 +950,9 @@ def lower(dev: R.Device, stores: List[Store], arena: ArenaMap, row_shard=None, f
             from .lower_generic import generic_statement
             stmt = generic_statement(dev, st, arena, sid)
         group = [st]
+        if merge and stmt.kind == "ew_stream" and last is not None and last.kind == "ew_stream" and last.try_merge(stmt):
+            groups[-1].append(st)           # the same tiles, read once for both stores
+            continue
         if FUSE_ROW_RESULTS and stmt.kind == "row_program" and not stmt.args.out_per_row:
             # ... and per-row results stored just before it
             while plan.statements and per_row_program(plan.statements[-1]) and stmt.try_absorb(groups[-1][0]):

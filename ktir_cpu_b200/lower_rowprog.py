@@ -26,7 +26,7 @@ import numpy as np
 from . import runtime as R
 from .dtypes import bytes_per_elem
 from .lower import (F_DT, ArenaMap, Footprint, Statement, _VM_BIN, _VM_UN, _access_offsets, _copy_args,
-                    _order_item_table, _points, strip_views, tile_geom)
+                    _order_item_table, _points, _runs_overlap, strip_views, tile_geom)
 from .trace import Access, Node, Store, Unsupported
 
 _RED_OPS = {"arith.addf": "add", "arith.maximumf": "max", "arith.maxnumf": "maxnum", "arith.maxf": "max"}
@@ -662,17 +662,6 @@ class RowProgramStatement(Statement):
 
     def bytes_moved(self):
         return self._bytes
-
-
-def _runs_overlap(s0, e0, s1, e1) -> bool:
-    """True if some run [s0, e0) meets some run [s1, e1)."""
-    if s0.min() >= e1.max() or s1.min() >= e0.max():
-        return False
-    order = np.argsort(s1, kind="stable")
-    s1, e1 = s1[order], np.maximum.accumulate(e1[order])
-    k = np.searchsorted(s1, e0, side="left") - 1          # last run of the second set that starts before each e0
-    ok = k >= 0
-    return bool((e1[k[ok]] > s0[ok]).any())
 
 
 def try_lower_row_program(dev, store: Store, arena: ArenaMap, stmt_id: int):

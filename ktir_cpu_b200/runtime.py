@@ -22,6 +22,10 @@ VM_OPS = ["MOV", "CONST", "ADD", "SUB", "MUL", "DIV", "MAX", "MAXNUM", "MIN", "M
           "EXP", "LOG", "LOG2", "SQRT", "RSQRT", "TANH", "SIN", "COS", "FMA"]
 VM = {n: i for i, n in enumerate(VM_OPS)}
 VM_ROUND16 = 0x100
+VM_EXTRA = {"CSEL": len(VM_OPS), "RSQRT_STEPS": len(VM_OPS) + 1, "ERF": len(VM_OPS) + 2}   # ktb_launch_ew_multi only
+# arith.cmpf predicates as the outcomes they hold for: less 1, equal 2, greater 4, unordered 8
+CMP = dict(oeq=2, one=5, olt=1, ole=3, ogt=4, oge=6, ord=7, uno=8, true=15, false=0, une=13, ueq=10, ult=9, ule=11, ugt=12, uge=14)
+EW_MAX_OUT = 8
 VM_IMM_A, VM_IMM_B = 0x200, 0x400          # row-value programs: operand a / b is the op's immediate
 
 
@@ -45,6 +49,13 @@ class EwArgs(C.Structure):
                 ("rows", C.c_int32), ("cols", C.c_int32),
                 ("row_stride", C.c_int64 * (VM_MAX_IN + 1)), ("dtype", C.c_int32 * (VM_MAX_IN + 1)),
                 ("vector_ok", C.c_int32), ("program", VmProgram)]
+
+
+class EwMultiArgs(C.Structure):
+    _fields_ = [("arena", C.c_void_p), ("dev_item_offsets", C.c_void_p), ("n_items", C.c_int64),
+                ("rows", C.c_int32), ("cols", C.c_int32), ("n_in", C.c_int32), ("n_out", C.c_int32),
+                ("row_stride", C.c_int64 * (VM_MAX_IN + EW_MAX_OUT)), ("dtype", C.c_int32 * (VM_MAX_IN + EW_MAX_OUT)),
+                ("vector_ok", C.c_int32), ("reserved", C.c_int32), ("program", VmProgram * EW_MAX_OUT)]
 
 
 RP_MAX_RED, RP_MAX_SCAL, RP_MAX_SIDE = 3, 4, 2
@@ -188,6 +199,7 @@ SYMBOLS = {
     "ktb_set_copy_threads": (C.c_int, [C.c_int]),
     "ktb_copy_threads": (C.c_int, []),
     "ktb_launch_ew_stream": (C.c_int, [C.c_void_p, C.POINTER(EwArgs)]),
+    "ktb_launch_ew_multi": (C.c_int, [C.c_void_p, C.POINTER(EwMultiArgs)]),
     "ktb_launch_row_program": (C.c_int, [C.c_void_p, C.POINTER(RowProgArgs)]),
     "ktb_launch_row_program_any": (C.c_int, [C.c_void_p, C.POINTER(RowProgArgs)]),
     "ktb_launch_row_softmax": (C.c_int, [C.c_void_p, C.POINTER(SoftmaxArgs)]),

@@ -151,7 +151,9 @@ def _erf_tile(x: Node) -> Node:
     for k in (3, 2, 1, 0):
         inner = ew("arith.mulf", [t, ew("arith.addf", [c(_ERF_C[k]), inner])])
     e = ew("math.exp", [ew("arith.mulf", [ew("arith.negf", [a]), a])])
-    return ew("arith.mulf", [ew("math.sign", [x]), ew("arith.subf", [c(1.0), ew("arith.mulf", [inner, e])])])
+    root = ew("arith.mulf", [ew("math.sign", [x]), ew("arith.subf", [c(1.0), ew("arith.mulf", [inner, e])])])
+    root.attrs["steps_of"] = ("ERF", x)          # what the chain computes, for lowerings that have it as one op
+    return root
 
 
 @rule(*_MATH)
@@ -162,7 +164,9 @@ def _math_unary(tr, op, scope):
             return _erf_tile(a)
         if op.name == "math.rsqrt":
             # 1.0 / np.sqrt(x) on the tile dtype (ktir_cpu/ops/math_ops.py:38-41): two ops, two roundings
-            return ew("arith.divf", [const_node(1.0, (), a.dtype), ew("math.sqrt", [a])])
+            root = ew("arith.divf", [const_node(1.0, (), a.dtype), ew("math.sqrt", [a])])
+            root.attrs["steps_of"] = ("RSQRT_STEPS", a)
+            return root
         return ew(op.name, [a])
     if _MATH[op.name] is None or isinstance(a, np.ndarray):
         raise Unsupported(f"{op.name} on a scalar")
