@@ -462,6 +462,12 @@ typedef struct {
     int64_t kv_page_stride, kv_row_stride, kv_head_stride;
     float scale, m_init, l_init;
     int32_t kv_group;                          /* query heads per K/V head */
+    /* few query rows (seq_q * kv_group <= 32): `splits` pieces the context is cut into, and scratch to merge them in:
+       32-bit counters, 8 per K/V head, zero before the first launch (each launch leaves them so), padded to 256 bytes,
+       then per K/V head, piece and row 32 times 24 bytes.  Launches that share scratch must be ordered.  0 / NULL:
+       one CTA per query head, as for any number of rows. */
+    int32_t splits, reserved;
+    void* dev_scratch;
 } ktb_attn_args;
 int ktb_launch_attention_fwd(ktb_ctx* ctx, const ktb_attn_args* args);
 

@@ -174,6 +174,11 @@ def match_attention(value: Node):
                 causal=causal, cond=cond, m_init=m_init, l_init=l_init, tile=masked.shape)
 
 
+# Query rows that share a K/V head, up to which the context is cut into pieces and spread over the SMs, and the CTAs that
+# makes (one per SM of the B200).
+DECODE_ROWS, DECODE_CTAS = 32, 148
+
+
 class AttentionStatement(Statement):
     kind = "attention_fwd"
 
@@ -292,6 +297,18 @@ class AttentionStatement(Statement):
         a.kv_page_stride, a.kv_row_stride, a.kv_head_stride = kview.strides[0], kview.strides[1], kview.strides[2]
         a.scale, a.m_init, a.l_init = m["scale"], m["m_init"], m["l_init"]
         self.device_arrays = []
+        kv_heads, q_rows = heads // grp, seq_q * grp
+        if q_rows <= DECODE_ROWS and heads % grp == 0:
+            seen = min(T * tn, seq_q + delta) if m["causal"] else T * tn
+            a.splits = max(1, min(-(-seen // 64), DECODE_CTAS // kv_heads))
+            if a.splits > 4:                      # whole clusters of four pieces; below that of 2^n
+                a.splits -= a.splits % 4
+            else:
+                a.splits = 1 << (a.splits.bit_length() - 1)
+            counters = (kv_heads * 8 * 4 + 255) // 256 * 256
+            a.dev_scratch = dev.alloc(counters + kv_heads * a.splits * q_rows * 32 * 24)
+            dev.memset(a.dev_scratch, 0, counters)
+            self.device_arrays = [a.dev_scratch]
         vis = np.minimum(T * tn, np.arange(seq_q) + 1 + delta) if m["causal"] else np.full(seq_q, T * tn)
         self.flops = int(4 * heads * hd * vis.sum())
         self._bytes = hd * 2 * (2 * heads * seq_q + 2 * ngrp * min(T, n_pages) * tn)

@@ -129,7 +129,8 @@ class AttnArgs(C.Structure):
                 ("q_row_stride", C.c_int64), ("q_head_stride", C.c_int64),
                 ("o_row_stride", C.c_int64), ("o_head_stride", C.c_int64),
                 ("kv_page_stride", C.c_int64), ("kv_row_stride", C.c_int64), ("kv_head_stride", C.c_int64),
-                ("scale", C.c_float), ("m_init", C.c_float), ("l_init", C.c_float), ("kv_group", C.c_int32)]
+                ("scale", C.c_float), ("m_init", C.c_float), ("l_init", C.c_float), ("kv_group", C.c_int32),
+                ("splits", C.c_int32), ("reserved", C.c_int32), ("dev_scratch", C.c_void_p)]
 
 
 G_MAXDIM = 6
@@ -410,6 +411,9 @@ class PlanOnlyDevice:
         return 0
 
     def free(self, ptr: int):
+        pass
+
+    def memset(self, ptr: int, value: int, nbytes: int):
         pass
 
     def upload(self, arr) -> int:

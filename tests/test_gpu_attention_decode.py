@@ -1,0 +1,73 @@
+"""Attention of a few query rows over a longer context: the kernel that cuts the context into pieces, against the oracle
+(the bars of the attention tests: P is rounded to f16 before P V, 2^-11 of each weight)."""
+import numpy as np
+import pytest
+
+from ktir_cpu_b200 import KTIRInterpreter, kernels as K, runtime as R
+from ktir_cpu_b200.interpreter import Session
+from ktir_cpu_b200.parser import KTIRParser
+from oracle.numpy_interp import OracleInterpreter
+
+
+def _case(tokens, before, heads, kv_heads, page, seed=0):
+    rng = np.random.default_rng(seed)
+    nb = -(-(before + tokens) // page)
+    f = lambda *s: rng.standard_normal(s, dtype=np.float32).astype(np.float16)     # noqa: E731
+    kw = dict(output_ptr=np.zeros((tokens, heads, 128), np.float16), query_ptr=f(tokens, heads, 128),
+              key_cache_ptr=f(nb, page, kv_heads, 128), value_cache_ptr=f(nb, page, kv_heads, 128),
+              block_tables_ptr=rng.permutation(nb).astype(np.int32).reshape(1, -1), cur_batch_start_index=0,
+              block_table_offset=0, num_tiles=nb, context_len=before, scale=np.float32(1 / np.sqrt(128)))
+    return K.paged_attention(tokens, before + tokens, heads, kv_heads, 128, page, tokens), kw
+
+
+# (tokens, positions before, query heads, K/V heads, page): one piece; pieces that end inside a page; an odd number of
+# 32-row pages; 16 rows, 17 (the second tile of rows), 32; head counts that are no power of two; one piece per head
+# and several waves; a long context in whole clusters with the last merge
+CASES = [(1, 0, 4, 4, 64), (1, 63, 2, 2, 64), (1, 64, 8, 1, 128), (3, 92, 4, 2, 32), (16, 130, 2, 2, 64), (17, 300, 1, 1, 128),
+         (4, 1000, 16, 2, 32), (2, 700, 9, 3, 64), (1, 65, 160, 160, 64), (1, 6000, 8, 1, 128), (32, 200, 3, 3, 32)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tokens,before,heads,kv_heads,page", CASES)
+def test_decode_matches_the_oracle(tokens, before, heads, kv_heads, page, build_lib):
+    src, kw = _case(tokens, before, heads, kv_heads, page)
+    gpu = KTIRInterpreter()
+    gpu.load(src)
+    first = gpu.execute_function("paged_attention_kernel", **kw)["output_ptr"]
+    again = gpu.execute_function("paged_attention_kernel", **kw)["output_ptr"]      # (the counters are back at zero)
+    st, = [s for sess in gpu._sessions.values() for s in sess.plan.statements]
+    assert st.kind == "attention_fwd" and st.args.splits >= 1 and st.args.dev_scratch
+    gpu.close()
+    ora = OracleInterpreter()
+    ora.load(src)
+    want = ora.execute_function("paged_attention_kernel", **kw)["output_ptr"]
+    np.testing.assert_allclose(first.astype(np.float32), want.astype(np.float32), rtol=1e-2, atol=2e-3)
+    np.testing.assert_array_equal(first, again)
+
+
+@pytest.mark.gpu
+def test_negative_page_is_reported(build_lib):
+    src, kw = _case(1, 500, 4, 2, 64)
+    kw["block_tables_ptr"][0, 3] = -7
+    gpu = KTIRInterpreter()
+    gpu.load(src)
+    with pytest.raises(IndexError, match="-7 is negative"):
+        gpu.execute_function("paged_attention_kernel", **kw)
+    kw["block_tables_ptr"][0, 3] = 3
+    gpu.execute_function("paged_attention_kernel", **kw)
+    gpu.close()
+
+
+@pytest.mark.parametrize("tokens,before,heads,kv_heads,splits", [(1, 8191, 64, 8, 16), (1, 60, 8, 8, 1), (4, 300, 32, 4, 4), (1, 5000, 2, 1, 76),
+                                                                 (1, 4000, 160, 160, 1), (1, 9999, 74, 74, 2), (33, 4000, 1, 1, 0)])
+def test_pieces_fill_clusters_and_no_more_than_the_context(tokens, before, heads, kv_heads, splits):
+    nb = -(-(before + tokens) // 64)
+    src = K.paged_attention(tokens, before + tokens, heads, kv_heads, 128, 64, tokens)
+    f16 = np.dtype(np.float16)
+    t = [("output_ptr", (tokens, heads, 128), f16), ("query_ptr", (tokens, heads, 128), f16), ("key_cache_ptr", (nb, 64, kv_heads, 128), f16),
+         ("value_cache_ptr", (nb, 64, kv_heads, 128), f16), ("block_tables_ptr", (1, nb), np.dtype(np.int32))]
+    s = Session(R.PlanOnlyDevice(), KTIRParser().parse_module(src).get_function("paged_attention_kernel"), t,
+                dict(cur_batch_start_index=0, block_table_offset=0, num_tiles=nb, context_len=before, scale=np.float32(0.1)), arena_ptr=0)
+    a = s.plan.statements[0].args
+    assert a.splits == splits and kv_heads * max(a.splits, 1) <= max(148, kv_heads)
+    assert a.splits < 4 or a.splits % 4 == 0
