@@ -435,6 +435,10 @@ typedef struct {
     int64_t lda, ldb, ldc;         /* elements */
     float c_init;                  /* constant initial value of the accumulator (usually 0) */
     int32_t reserved;
+    /* few tiles: tile_n = 64 or 128 asks for 128 x tile_n tiles with K cut into split_k (1, 2, 4) ranges, each a CTA;
+       0: 256 x 256 tiles on CTA pairs (128 x 128 / 256 for a single row tile).  The order of a sum depends on split_k
+       and K only. */
+    int32_t tile_n, split_k;
 } ktb_gemm_args;
 int ktb_launch_gemm_f16(ktb_ctx* ctx, const ktb_gemm_args* args);
 

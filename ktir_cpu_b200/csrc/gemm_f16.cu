@@ -17,6 +17,8 @@
 // work).  When at most G / 2 tiles are left over, each is cut into its left and right half
 // (128 x BN/2) and the halves go to twice as many SMs: the tail takes about half a tile time, the
 // k order of every sum is unchanged (results do not depend on how the tiles were dealt out).
+#include <cooperative_groups.h>
+
 #include "tc_common.cuh"
 
 #define GEMM_BM 128
@@ -368,6 +370,180 @@ ktb_gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     if (warp == 1) tc_tmem_dealloc_pair(tmem_base, 2 * GEMM2_BN);
 }
 
+// ---- products with few tiles ---------------------------------------------------------------------
+// One 128 x BN tile and one of S ranges of K per CTA, the S CTAs of a tile in a cluster: a product of few rows (a
+// decode batch) or of small extents has too few 256 x 256 tiles for 148 SMs, and each walks all of K.  Loads as in
+// ktb_gemm_f16_kernel; A tiles hold no more rows than the matrix has (the accumulator rows beyond are never read).  The
+// f32 partial tiles meet in shared memory: every CTA adds up a 1 / S-th of the rows over its cluster, range after range,
+// so a sum's order depends on S and K alone, not on the tile that it falls into.
+// Bound by the chain load -> MMA -> exchange of one tile, next to reading B.  f16 [64, 2880] x [2880, 5760]: 14.6 us
+// (5.3 at the measured copy rate), 20.6 on 23 tiles of 256 columns; [16, 4096] x [4096, 512]: 10.3, 24.6 before.
+template <int BN>
+struct GemmFew {
+    static constexpr int STAGES = BN == 64 ? 8 : 6;
+    static constexpr int B_BYTES = GEMM_BK * BN * 2;
+    static constexpr int PITCH = BN + 4;                 // floats per row of the partial tile
+    static constexpr size_t RING = (size_t)STAGES * (GEMM_A_STAGE_BYTES + B_BYTES);
+    static constexpr size_t SMEM = RING + 1024 + 256;
+    static_assert(RING >= (size_t)GEMM_BM * PITCH * 4, "the partial tile takes the ring's place");
+};
+
+template <int BN>
+__global__ void __launch_bounds__(GEMM_THREADS, 1)
+ktb_gemm_f16_few_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const ktb_gemm_args a,
+                        int a_rows, int tiles_n, ktb_status* st) {
+    using Cfg = GemmFew<BN>;
+    constexpr int S = Cfg::STAGES;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    uint8_t* sA = smem;
+    uint8_t* sB = smem + (size_t)S * GEMM_A_STAGE_BYTES;
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + Cfg::RING);
+    uint64_t* empty = full + S;
+    uint64_t* done = empty + S;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    // (through a shuffle, so that the compiler knows the warp index is the same in all lanes)
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    const int parts = a.split_k, part = blockIdx.x % parts, tile = blockIdx.x / parts;
+    const int m0 = tile / tiles_n * GEMM_BM, n0 = tile % tiles_n * BN;
+    const int KT = (a.K + GEMM_BK - 1) / GEMM_BK;
+    const int k0 = (int)((int64_t)KT * part / parts), k1 = (int)((int64_t)KT * (part + 1) / parts);
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < S; ++i) {
+            tc_mbar_init(&full[i], 1);
+            tc_mbar_init(&empty[i], 1);
+        }
+        tc_mbar_init(done, 1);
+        *abort_flag = 0;
+        tc_fence_barrier_init();
+    }
+    __syncthreads();
+    if (warp == 1) tc_tmem_alloc(tmem_slot, BN);
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+
+    if (warp == 0) {
+        if (lane == 0) {
+            tc_prefetch_tmap(&map_a);
+            tc_prefetch_tmap(&map_b);
+            for (int i = 0; i < k1 - k0; ++i) {
+                const int stage = i % S;
+                if (!tc_mbar_wait(&empty[stage], ((i / S) & 1) ^ 1, abort_flag, st, 51)) break;
+                tc_mbar_expect_tx(&full[stage], a_rows * GEMM_BK * 2 + Cfg::B_BYTES);
+                tc_tma_load_2d(sA + (size_t)stage * GEMM_A_STAGE_BYTES, &map_a, &full[stage], (k0 + i) * GEMM_BK, m0);
+#pragma unroll
+                for (int j = 0; j < BN / 64; ++j)
+                    tc_tma_load_2d(sB + (size_t)stage * Cfg::B_BYTES + (size_t)j * (GEMM_BK * 128), &map_b, &full[stage], n0 + j * 64,
+                                   (k0 + i) * GEMM_BK);
+            }
+        }
+    } else if (warp == 1) {
+        // the warp runs converged and one elected lane issues: descriptors stay in uniform registers, and an MMA takes 9
+        // cycles of issue instead of the 44 and more under `if (lane == 0)`, which set the pace of a step here (0.33 us
+        // whatever the tile; 0.20 this way)
+        const uint32_t lead = tc_elect_one();
+        const uint32_t idesc = tc_idesc_f16(GEMM_BM, BN, 0, 1);
+        const uint64_t ad0 = tc_smem_desc(tc_smem_u32(sA), 16, 1024), bd0 = tc_smem_desc(tc_smem_u32(sB), GEMM_BK * 128, 1024);
+        bool ok = true;
+        for (int i = 0, phase = 0; i < k1 - k0 && ok; phase ^= 1) {
+#pragma unroll
+            for (int stage = 0; stage < S; ++stage, ++i) {
+                if (i >= k1 - k0) break;
+                ok = __all_sync(0xffffffffu, tc_mbar_wait(&full[stage], phase, abort_flag, st, 52)) != 0;
+                if (!ok) break;
+                tc_fence_after_sync();
+#pragma unroll
+                for (int kk = 0; kk < GEMM_BK / 16; ++kk)
+                    tc_mma_f16_p(tmem, ad0 + (uint32_t)((stage * GEMM_A_STAGE_BYTES + kk * 32) >> 4),
+                                 bd0 + (uint32_t)((stage * Cfg::B_BYTES + kk * 2048) >> 4), idesc, (i | kk) != 0, lead);
+                tc_mma_commit_p(&empty[stage], lead);
+            }
+        }
+        if (ok) tc_mma_commit_p(done, lead);
+    } else {
+        // (the last MMA has completed, so every load has landed and been read: the ring is free)
+        const bool ok = __all_sync(0xffffffffu, tc_mbar_wait(done, 0, abort_flag, st, 53)) != 0;
+        tc_fence_after_sync();
+        const int q = warp & 3;                          // TMEM lane quadrant this warp may read
+        float* row = reinterpret_cast<float*>(smem) + (q * 32 + lane) * Cfg::PITCH;
+        if (ok)
+#pragma unroll 1
+            for (int c = 0; c < BN; c += 32) {
+                uint32_t r[32];
+                tc_tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + c, r);
+                tc_tmem_ld_wait();
+#pragma unroll
+                for (int i = 0; i < 32; i += 4)
+                    *reinterpret_cast<uint4*>(row + c + i) = make_uint4(r[i], r[i + 1], r[i + 2], r[i + 3]);
+            }
+    }
+    tc_fence_before_sync();
+    __syncthreads();
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    if (parts > 1) cl.sync();
+    // rows part, part + S, ... of the tile, eight columns per thread and step
+    const int rows = a.M - m0 < GEMM_BM ? a.M - m0 : GEMM_BM;
+    const bool f16 = a.c_dtype == KTB_F16;
+    if (*abort_flag == 0)
+        for (int e = threadIdx.x; e < (rows - part + parts - 1) / parts * (BN / 8); e += GEMM_THREADS) {
+            const int row = e / (BN / 8) * parts + part, col = e % (BN / 8) * 8;
+            if (n0 + col >= a.N) continue;
+            float4 x = make_float4(0.f, 0.f, 0.f, 0.f), y = x;
+            for (int p = 0; p < parts; ++p) {
+                float* at = reinterpret_cast<float*>(smem) + row * Cfg::PITCH + col;
+                const float4* src = reinterpret_cast<const float4*>(parts > 1 ? cl.map_shared_rank(at, p) : at);
+                const float4 u = src[0], v = src[1];
+                if (p == 0) {
+                    x = u;
+                    y = v;
+                } else {
+                    x.x += u.x; x.y += u.y; x.z += u.z; x.w += u.w;
+                    y.x += v.x; y.y += v.y; y.z += v.z; y.w += v.w;
+                }
+            }
+            const float ci = a.c_init;
+            x.x += ci; x.y += ci; x.z += ci; x.w += ci;
+            y.x += ci; y.y += ci; y.z += ci; y.w += ci;
+            const int64_t off = a.c_off + (int64_t)(m0 + row) * a.ldc + n0 + col;
+            if (f16) {
+                __half2 h[4] = {__floats2half2_rn(x.x, x.y), __floats2half2_rn(x.z, x.w), __floats2half2_rn(y.x, y.y), __floats2half2_rn(y.z, y.w)};
+                *reinterpret_cast<uint4*>(reinterpret_cast<__half*>(a.arena) + off) = *reinterpret_cast<const uint4*>(h);
+            } else {
+                float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(a.arena) + off);
+                dst[0] = x;
+                dst[1] = y;
+            }
+        }
+    if (parts > 1) cl.sync();                            // peers may still read this CTA's shared memory
+    if (warp == 1) tc_tmem_dealloc(tmem, BN);
+}
+
+template <int BN>
+static int launch_gemm_few(ktb_ctx* ctx, const ktb_gemm_args& a, const CUtensorMap& ma, const CUtensorMap& mb, int a_rows) {
+    using Cfg = GemmFew<BN>;
+    const int tiles_m = (a.M + GEMM_BM - 1) / GEMM_BM, tiles_n = (a.N + BN - 1) / BN;
+    KTB_CUDA(ctx, cudaFuncSetAttribute(ktb_gemm_f16_few_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::SMEM));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(tiles_m * tiles_n * a.split_k));
+    cfg.blockDim = dim3(GEMM_THREADS);
+    cfg.dynamicSmemBytes = Cfg::SMEM;
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = a.split_k;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    KTB_CUDA(ctx, cudaLaunchKernelEx(&cfg, ktb_gemm_f16_few_kernel<BN>, ma, mb, a, a_rows, tiles_n, ctx->dev_status));
+    KTB_CHECK_LAUNCH(ctx, "ktb_gemm_f16_few_kernel");
+    return KTB_OK;
+}
+
 template <int BN>
 static int launch_gemm(ktb_ctx* ctx, const ktb_gemm_args& a, const CUtensorMap& ma, const CUtensorMap& mb,
                        const CUtensorMap& mc) {
@@ -409,12 +585,18 @@ extern "C" int ktb_launch_gemm_f16(ktb_ctx* ctx, const ktb_gemm_args* args) {
     if (a.c_dtype != KTB_F16 && a.c_dtype != KTB_F32) return ktb_fail(ctx, KTB_E_UNSUPPORTED, "gemm_f16", "C must be f16 or f32");
     if ((a.N % 32) || (a.K % 8) || (a.lda % 8) || (a.ldb % 8) || (a.ldc % 8) || (a.a_off % 8) || (a.b_off % 8) || (a.c_off % 8))
         return ktb_fail(ctx, KTB_E_UNSUPPORTED, "gemm_f16", "N must be a multiple of 32; K, leading dims and offsets multiples of 8");
+    if ((a.tile_n != 0 && a.tile_n != 64 && a.tile_n != 128) || (a.tile_n && a.split_k != 1 && a.split_k != 2 && a.split_k != 4))
+        return ktb_fail(ctx, KTB_E_ARG, "gemm_f16", "tile_n must be 0, 64 or 128 and split_k then 1, 2 or 4");
+    if (a.tile_n && (a.K + GEMM_BK - 1) / GEMM_BK < a.split_k)
+        return ktb_fail(ctx, KTB_E_ARG, "gemm_f16", "every range of K takes at least one step of 64");
+    // rows of an A tile: all that there are when the product is less than a tile high (whole swizzle groups of 8)
+    const int a_rows = a.tile_n && a.M < GEMM_BM ? (a.M + 7) & ~7 : GEMM_BM;
     CUtensorMap ma, mb, mc;
     __half* base = reinterpret_cast<__half*>(a.arena);
     {
         const uint64_t dims[2] = {(uint64_t)a.K, (uint64_t)a.M};
         const uint64_t str[1] = {(uint64_t)a.lda * 2};
-        const uint32_t box[2] = {GEMM_BK, GEMM_BM};
+        const uint32_t box[2] = {GEMM_BK, (uint32_t)a_rows};
         if (!tc_make_map_f16(&ma, base + a.a_off, 2, dims, str, box)) return ktb_fail(ctx, KTB_E_CUDA, "gemm_f16", "cuTensorMapEncodeTiled(A) failed");
     }
     {
@@ -423,6 +605,8 @@ extern "C" int ktb_launch_gemm_f16(ktb_ctx* ctx, const ktb_gemm_args* args) {
         const uint32_t box[2] = {64, GEMM_BK};
         if (!tc_make_map_f16(&mb, base + a.b_off, 2, dims, str, box)) return ktb_fail(ctx, KTB_E_CUDA, "gemm_f16", "cuTensorMapEncodeTiled(B) failed");
     }
+    if (a.tile_n == 64) return launch_gemm_few<64>(ctx, a, ma, mb, a_rows);
+    if (a.tile_n == 128) return launch_gemm_few<128>(ctx, a, ma, mb, a_rows);
     {
         // C as the epilogue stores it: 32 rows x 128 bytes per tile store
         const bool f16 = a.c_dtype == KTB_F16;

@@ -124,7 +124,7 @@ class Session:
             if latency:
                 self.latency_records = tracer.latency.records
             self.n_cores = tracer.ncores
-            row_shard = None
+            row_shard = whole = None
             if shard is not None and shard[1] > 1:
                 from .sharded import core_slice, needs_row_ownership
                 if needs_row_ownership(stores):
@@ -132,12 +132,16 @@ class Session:
                 else:
                     # a core of another rank may read or overlap what a core of this rank writes: the
                     # whole grid must pass the sequential-order check, not just this rank's slice
-                    lower(R.PlanOnlyDevice(), stores, self.arena_map, fused=fused)
+                    whole = lower(R.PlanOnlyDevice(), stores, self.arena_map, fused=fused)
                     part = Tracer(func, scalars, ptrs, core_range=core_slice(tracer.ncores, *shard))
                     part.arena = self.arena_map
                     stores = part.run()
             try:
                 self.plan: Plan = lower(dev, stores, self.arena_map, row_shard=row_shard, fused=fused)
+                if whole is not None:      # a rank's part of a product adds up K as the whole would
+                    for mine, full in zip(self.plan.statements, whole.statements):
+                        if mine.kind == full.kind == "gemm_f16":
+                            mine.args.tile_n, mine.args.split_k = full.args.tile_n, full.args.split_k
             except CoreOrderHazard:
                 if shard is not None and shard[1] > 1:
                     raise

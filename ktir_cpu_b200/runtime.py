@@ -117,7 +117,7 @@ class GemmArgs(C.Structure):
     _fields_ = [("arena", C.c_void_p), ("a_off", C.c_int64), ("b_off", C.c_int64), ("c_off", C.c_int64),
                 ("M", C.c_int32), ("N", C.c_int32), ("K", C.c_int32), ("c_dtype", C.c_int32),
                 ("lda", C.c_int64), ("ldb", C.c_int64), ("ldc", C.c_int64),
-                ("c_init", C.c_float), ("reserved", C.c_int32)]
+                ("c_init", C.c_float), ("reserved", C.c_int32), ("tile_n", C.c_int32), ("split_k", C.c_int32)]
 
 
 class AttnArgs(C.Structure):

@@ -1,0 +1,75 @@
+"""Products with few tiles: 128 x 64 / 128 x 128 tiles, K in ranges that a cluster adds up."""
+import numpy as np
+import pytest
+
+from ktir_cpu_b200 import KTIRInterpreter, kernels as K, runtime as R
+from ktir_cpu_b200.interpreter import Session
+from ktir_cpu_b200.lower_mm import few_tiles
+from ktir_cpu_b200.parser import KTIRParser
+
+
+def _run(M, N, Kd, bm, bn, bk, f32, plan=None):
+    rng = np.random.default_rng(M + N + Kd)
+    a, b = (rng.uniform(-1, 1, s).astype(np.float16) for s in ((M, Kd), (Kd, N)))
+    cores = next(c for c in (8, 4, 3, 2, 1) if (M // bm) * (N // bn) % c == 0)
+    it = KTIRInterpreter()
+    it.load(K.tiled_matmul(M, N, Kd, bm, bn, bk, cores, f32))
+    kw = dict(a_ptr=a, b_ptr=b, c_ptr=np.full((M, N), 9, np.float16))
+    sess, _ = it.session("matmul_kernel", **kw)
+    args = sess.plan.statements[0].args
+    if plan is not None:
+        args.tile_n, args.split_k = plan
+    got = it.execute_function("matmul_kernel", **kw)["c_ptr"]
+    it.close()
+    return got, a.astype(np.float64) @ b.astype(np.float64), (args.tile_n, args.split_k)
+
+
+# (M, N, K, bm, bn, bk): rows that do not fill a tile or its last one, N that ends inside a tile of 64 and of 128, K that
+# ends inside a step of 64 and ranges of unequal length, one step for four ranges, a single tile
+SHAPES = [(16, 64, 512, 16, 64, 64), (8, 32, 64, 8, 32, 64), (24, 96, 200, 24, 32, 40), (64, 160, 1032, 32, 32, 8), (144, 96, 320, 16, 32, 64),
+          (128, 256, 256, 64, 64, 64), (272, 352, 712, 16, 32, 8), (300, 128, 4096, 20, 64, 64)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M,N,Kd,bm,bn,bk", SHAPES)
+def test_every_tile_and_split_gives_the_product(M, N, Kd, bm, bn, bk, build_lib):
+    """f32 sums of K products of magnitude below 1 (error K 2^-24 at most) and one rounding to f16 (2^-11)."""
+    base = None
+    for plan in [(t, s) for t in (64, 128) for s in (1, 2, 4) if -(-Kd // 64) >= s] + [(0, 0)]:
+        got, want, _ = _run(M, N, Kd, bm, bn, bk, True, plan)
+        np.testing.assert_allclose(got.astype(np.float64), want, rtol=2.0 ** -11, atol=Kd * 2.0 ** -24 + 2.0 ** -12, err_msg=str(plan))
+        if plan[1] in (0, 1):        # K in one range: the same sums whatever the tile
+            base = got if base is None else base
+            np.testing.assert_array_equal(got, base, err_msg=str(plan))
+
+
+@pytest.mark.gpu
+def test_f16_accumulator_form_takes_it_too(build_lib):
+    got, want, plan = _run(64, 512, 2880, 64, 64, 64, False)
+    assert plan == (64, 4)
+    np.testing.assert_allclose(got.astype(np.float64), want, rtol=2e-2, atol=2e-1)
+
+
+def test_rule():
+    assert few_tiles(4096, 4096, 4096) == (0, 0) and few_tiles(2048, 2048, 512) == (0, 0)
+    assert few_tiles(64, 5760, 2880) == (64, 1) and few_tiles(64, 4096, 4096) == (64, 2) and few_tiles(16, 512, 4096) == (64, 4)
+    assert few_tiles(1536, 1536, 2048) == (128, 1) and few_tiles(256, 256, 256) == (64, 1)
+    assert few_tiles(848, 1408, 352) == (0, 0) and few_tiles(848, 1408, 2048) == (128, 1)
+    for M in (1, 100, 128, 1000, 2304):
+        for N in (32, 512, 4096):
+            for Kd in (8, 64, 1000, 8192):
+                t, s = few_tiles(M, N, Kd)
+                assert (t, s) == (0, 0) or (t in (64, 128) and s in (1, 2, 4) and (s == 1 or -(-Kd // 64) >= 4 * s))
+
+
+def test_a_ranks_part_adds_up_like_the_whole():
+    """Cores of one rank cover fewer rows, but K is cut as for the whole product."""
+    src = K.tiled_matmul(256, 512, 4096, 64, 64, 64, 8, True)
+    f16 = np.dtype(np.float16)
+    t = [("a_ptr", (256, 4096), f16), ("b_ptr", (4096, 512), f16), ("c_ptr", (256, 512), f16)]
+    func = KTIRParser().parse_module(src).get_function("matmul_kernel")
+    whole = Session(R.PlanOnlyDevice(), func, t, {}, arena_ptr=0).plan.statements[0].args
+    for rank in range(4):
+        part = Session(R.PlanOnlyDevice(), func, t, {}, arena_ptr=0, shard=(rank, 4)).plan.statements[0].args
+        assert part.M == 64 and (part.tile_n, part.split_k) == (whole.tile_n, whole.split_k)
+    assert whole.split_k == 4
