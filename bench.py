@@ -287,7 +287,7 @@ class Attention(Workload):
 class LayerNorm(Workload):
     """The reference's layer-norm example (examples/triton-ktir/layernorm_fwd_ktir.mlir: f16 throughout, rows
     walked in column blocks, Mean and Rstd kept per row) at 4096 rows of its 8192 columns."""
-    name, func, kernel = "layernorm", "_layer_norm_fwd_fused", "ktb_row_norm_h_kernel"
+    name, func, kernel = "layernorm", "_layer_norm_fwd_fused", "ktb_row_norm_any_kernel"
     ROWS, COLS, BLOCK, CORES = 4096, 8192, 1024, 32
     units_per_step = ROWS * COLS
     algo_per_step = 4 * ROWS * COLS * 2 + 2 * ROWS * 2          # X, W, B read, Y written; Mean and Rstd
