@@ -468,9 +468,11 @@ typedef struct {
     int32_t kv_group;                          /* query heads per K/V head */
     /* few query rows (seq_q * kv_group <= 32): `splits` pieces the context is cut into, and scratch to merge them in:
        32-bit counters, 8 per K/V head, zero before the first launch (each launch leaves them so), padded to 256 bytes,
-       then per K/V head, piece and row 32 times 24 bytes.  Launches that share scratch must be ordered.  0 / NULL:
-       one CTA per query head, as for any number of rows. */
-    int32_t splits, reserved;
+       then per K/V head, piece and row 32 times 24 bytes.  scratch_heads: the K/V heads that the scratch is laid out for,
+       the same for every launch that shares it (a launch over some of the heads, say) and no less than the launch has;
+       0: those of this launch.  Launches that share scratch must be ordered.  0 / NULL: one CTA per query head, as for
+       any number of rows. */
+    int32_t splits, scratch_heads;
     void* dev_scratch;
 } ktb_attn_args;
 int ktb_launch_attention_fwd(ktb_ctx* ctx, const ktb_attn_args* args);

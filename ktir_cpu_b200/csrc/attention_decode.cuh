@@ -42,9 +42,10 @@ static __device__ __forceinline__ void ad_ldm4t(uint32_t addr, uint32_t (&r)[4])
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
 }
 
-// Scratch of one launch: a counter per K/V head and slice, then per head, cluster and group of four dims the partial
-// O, then its (max, sum).
-static __host__ __device__ __forceinline__ size_t ad_counter_bytes(int n) { return ((size_t)n * 4 + 255) & ~(size_t)255; }
+// Scratch: a counter per K/V head and slice, then per head, cluster and group of four dims the partial O, then its
+// (max, sum).  The counters outlive a launch, so where they end depends on the heads that the scratch is laid out for
+// and not on those of the launch: parts of a statement share one scratch with the whole of it.
+static __host__ __device__ __forceinline__ size_t ad_counter_bytes(int heads) { return ((size_t)heads * 32 + 255) & ~(size_t)255; }
 
 template <int MT>                        // tiles of 16 query rows
 __global__ void __launch_bounds__(AD_THREADS, 1)
@@ -305,7 +306,7 @@ ktb_attention_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __g
     const int rank = piece % cluster, clusters = a.splits / cluster, kv_heads = gridDim.x / a.splits;
     const int per = (rows * 32 + cluster - 1) / cluster;
     const int e0 = rank * per, e1 = e0 + per < rows * 32 ? e0 + per : rows * 32;
-    float4* part_o = reinterpret_cast<float4*>(reinterpret_cast<uint8_t*>(a.dev_scratch) + ad_counter_bytes(kv_heads * cluster));
+    float4* part_o = reinterpret_cast<float4*>(reinterpret_cast<uint8_t*>(a.dev_scratch) + ad_counter_bytes(a.scratch_heads ? a.scratch_heads : kv_heads));
     float2* part_ml = reinterpret_cast<float2*>(part_o + (size_t)a.splits / cluster * kv_heads * rows * 32);
     auto merge = [&](int n_parts, auto ml_of, auto o_of, float4& o, float& mx, float& sum) {
         mx = -INFINITY;

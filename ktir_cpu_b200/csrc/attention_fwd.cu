@@ -622,6 +622,8 @@ extern "C" int ktb_launch_attention_fwd(ktb_ctx* ctx, const ktb_attn_args* args)
     // Up to 32 query rows per K/V head, and scratch to merge pieces of the context in: the decode kernel.
     // (The line: 32 tokens of 32 heads over 544 positions cost 12.4 us either way, 16 over 2064 14.4 against 28.7.)
     const bool decode = a.splits > 0 && a.dev_scratch && a.heads % kvg == 0 && (int64_t)a.seq_q * kvg <= AD_MAX_ROWS;
+    if (decode && a.scratch_heads != 0 && a.scratch_heads < a.heads / kvg)
+        return ktb_fail(ctx, KTB_E_ARG, "attention_fwd", "scratch laid out for fewer K/V heads than the launch has");
     const uint32_t box_rows = decode && a.page > AD_ROWS ? AD_ROWS : (uint32_t)a.page;
     for (int which = 0; which < 2; ++which) {
         const uint64_t dims[4] = {AT_D, (uint64_t)((a.heads + kvg - 1) / kvg), (uint64_t)a.page, (uint64_t)a.n_pages_total};

@@ -305,6 +305,7 @@ class AttentionStatement(Statement):
                 a.splits -= a.splits % 4
             else:
                 a.splits = 1 << (a.splits.bit_length() - 1)
+            a.scratch_heads = kv_heads            # (parts of the statement keep it: their counters are the whole's)
             counters = (kv_heads * 8 * 4 + 255) // 256 * 256
             a.dev_scratch = dev.alloc(counters + kv_heads * a.splits * q_rows * 32 * 24)
             dev.memset(a.dev_scratch, 0, counters)

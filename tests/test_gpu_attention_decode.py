@@ -1,5 +1,7 @@
 """Attention of a few query rows over a longer context: the kernel that cuts the context into pieces, against the oracle
 (the bars of the attention tests: P is rounded to f16 before P V, 2^-11 of each weight)."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -71,3 +73,39 @@ def test_pieces_fill_clusters_and_no_more_than_the_context(tokens, before, heads
     a = s.plan.statements[0].args
     assert a.splits == splits and kv_heads * max(a.splits, 1) <= max(148, kv_heads)
     assert a.splits < 4 or a.splits % 4 == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kv_heads,group", [(17, 1), (18, 2), (8, 4), (32, 1)])
+def test_whole_and_parts_share_the_scratch(kv_heads, group, build_lib):
+    """Eight or more pieces (two clusters per head and slice, so the counters in scratch are used): launches over all
+    heads, over parts of them and over all again, on one scratch, give the same bits, those of the oracle's bar."""
+    src, kw = _case(1, 1200, kv_heads * group, kv_heads, 64)
+    gpu = KTIRInterpreter()
+    gpu.load(src)
+    sess, _ = gpu.session("paged_attention_kernel", **kw)
+    st, = sess.plan.statements
+    parts = [c.launch for c in st.split(st.bytes_moved() // 4)]
+    assert len(parts) == 4 and (st.args.splits >= 8 or kv_heads == 32)
+    for k, v in kw.items():
+        if isinstance(v, np.ndarray):
+            sess.upload(k, v)
+
+    def output(whole):
+        sess.upload("output_ptr", kw["output_ptr"])
+        if whole:
+            sess.run()
+        for name, args in [] if whole else parts:
+            args.arena = sess.arena
+            gpu.device.check(getattr(gpu.device.lib, name)(gpu.device.h, C.byref(args)))
+        out = sess.download("output_ptr")
+        gpu.device.sync()
+        return out.view(np.uint16)
+    got = [output(whole) for whole in (True, False, True, True, False, True)]
+    gpu.close()
+    for other in got[1:]:
+        np.testing.assert_array_equal(got[0], other)
+    ora = OracleInterpreter()
+    ora.load(src)
+    want = ora.execute_function("paged_attention_kernel", **kw)["output_ptr"]
+    np.testing.assert_allclose(got[0].view(np.float16).astype(np.float32), want.astype(np.float32), rtol=1e-2, atol=2e-3)
