@@ -309,6 +309,7 @@ class AttentionStatement(Statement):
             counters = (kv_heads * 8 * 4 + 255) // 256 * 256
             a.dev_scratch = dev.alloc(counters + kv_heads * a.splits * q_rows * 32 * 24)
             dev.memset(a.dev_scratch, 0, counters)
+            dev.sync()                            # (the context may be moved to another stream before the first run)
             self.device_arrays = [a.dev_scratch]
         vis = np.minimum(T * tn, np.arange(seq_q) + 1 + delta) if m["causal"] else np.full(seq_q, T * tn)
         self.flops = int(4 * heads * hd * vis.sum())

@@ -109,3 +109,22 @@ def test_whole_and_parts_share_the_scratch(kv_heads, group, build_lib):
     ora.load(src)
     want = ora.execute_function("paged_attention_kernel", **kw)["output_ptr"]
     np.testing.assert_allclose(got[0].view(np.float16).astype(np.float32), want.astype(np.float32), rtol=1e-2, atol=2e-3)
+
+
+def test_counters_are_zero_before_planning_returns():
+    """Tables are uploaded with a wait; the zeros of the merge counters too: the context may go to another stream between
+    planning and the first run, and the memset is queued on the one of the planning."""
+    calls = []
+
+    class Device(R.PlanOnlyDevice):
+        def memset(self, ptr, value, nbytes):
+            calls.append(("memset", value, nbytes))
+
+        def sync(self):
+            calls.append(("sync",))
+            return R.Status()
+    src, kw = _case(1, 2000, 8, 4, 64)
+    Session(Device(), KTIRParser().parse_module(src).get_function("paged_attention_kernel"),
+            [(k, v.shape, v.dtype) for k, v in kw.items() if isinstance(v, np.ndarray)],
+            {k: v for k, v in kw.items() if not isinstance(v, np.ndarray)}, arena_ptr=0)
+    assert calls == [("memset", 0, 256), ("sync",)]
