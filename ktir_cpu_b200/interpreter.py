@@ -138,10 +138,8 @@ class Session:
                     stores = part.run()
             try:
                 self.plan: Plan = lower(dev, stores, self.arena_map, row_shard=row_shard, fused=fused)
-                if whole is not None:      # a rank's part of a product adds up K as the whole would
-                    for mine, full in zip(self.plan.statements, whole.statements):
-                        if mine.kind == full.kind == "gemm_f16":
-                            mine.args.tile_n, mine.args.split_k = full.args.tile_n, full.args.split_k
+                if whole is not None:      # a rank's part adds up as the whole would
+                    self.plan.follow(whole, dev)
             except CoreOrderHazard:
                 if shard is not None and shard[1] > 1:
                     raise

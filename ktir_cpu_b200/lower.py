@@ -69,6 +69,7 @@ class Statement:
     kind = "?"
     device_arrays: List[int]
     launches = 1
+    origin: Tuple[int, ...] = ()           # of the store it was made for (``Store.origin``)
 
     def launch(self, dev: R.Device, arena_ptr: int):
         raise NotImplementedError
@@ -78,6 +79,10 @@ class Statement:
 
     def bytes_moved(self) -> int:
         return 0
+
+    def follow(self, whole: "Statement", dev: R.Device):
+        """Take over what decides the order of this statement's sums from ``whole``, the statement that the same store
+        became in the plan of the whole grid."""
 
     def split(self, piece_bytes: int):
         """Independent parts of this statement for pipelined execution (``pipeline.Chunk`` list:
@@ -814,6 +819,16 @@ class Plan:
         for s in self.statements:
             s.launch(dev, arena_ptr)
 
+    def follow(self, whole: "Plan", dev: R.Device):
+        """This plan covers some of the cores of ``whole``: its statements add up as those of the same stores there.
+        (By the store, not by position: which stores join a launch, and the order of the launches, depend on the bytes
+        that the cores at hand touch.)"""
+        full = {s.origin: s for s in whole.statements}
+        for s in self.statements:
+            w = full.get(s.origin)
+            if w is not None and w.kind == s.kind:
+                s.follow(w, dev)
+
     def written_ranges(self) -> List[Tuple[int, int]]:
         """Arena byte ranges the launches write, merged and sorted."""
         runs = []
@@ -949,6 +964,7 @@ def lower(dev: R.Device, stores: List[Store], arena: ArenaMap, row_shard=None, f
                 raise
             from .lower_generic import generic_statement
             stmt = generic_statement(dev, st, arena, sid)
+        stmt.origin = st.origin
         group = [st]
         if merge and stmt.kind == "ew_stream" and last is not None and last.kind == "ew_stream" and last.try_merge(stmt):
             groups[-1].append(st)           # the same tiles, read once for both stores

@@ -173,6 +173,10 @@ class GemmStatement(Statement):
         self.args.arena = arena_ptr
         dev.check(dev.lib.ktb_launch_gemm_f16(dev.h, C.byref(self.args)))
 
+    def follow(self, whole: "GemmStatement", dev: R.Device):
+        if self.args.K == whole.args.K:
+            self.args.tile_n, self.args.split_k = whole.args.tile_n, whole.args.split_k
+
     def split(self, piece_bytes: int):
         """Row blocks of C: block [m0, m1) needs the same rows of A and all of B."""
         from .lower import _copy_args

@@ -155,6 +155,7 @@ class Store:
     active: Optional[np.ndarray]   # bool mask over the iteration space, None = all
     seq: int = 0
     loop_path: Tuple[int, ...] = ()
+    origin: Tuple[int, ...] = ()   # which op of the function stores, in which iterations of the loops traced one by one
 
 
 @dataclass
@@ -188,6 +189,7 @@ class Tracer:
         self.unroll_loops = False       # trace every scf.for iteration by iteration (its stores become statements of their own)
         self.loop_path: List[int] = []
         self._loop_counter = 0
+        self.iterations: List[int] = []  # of the loops around the op being traced that are traced iteration by iteration
         self.latency = None            # a trace_latency.LatencyRecorder when the latency model is on
         self.lx = None                 # an lx.LXModel when scratchpad accounting is on
         self.arena = None              # a lower.ArenaMap: accesses are clipped to the allocation they start in

@@ -306,5 +306,5 @@ def _store(tr, op, scope):
         raise Unsupported("ktdp.store to a value that is not an access tile")
     tr.stores.append(Store(value, at, tuple(tr.axes),
                            None if tr.active is None else tr.active.copy(),
-                           len(tr.stores), tuple(tr.loop_path)))
+                           len(tr.stores), tuple(tr.loop_path), (id(op), *tr.iterations)))
     return None

@@ -478,7 +478,9 @@ def _for(tr: Tracer, op: Op, scope):
         inner[iv_name] = iv_bin(lambda a, b: a + b, lb, iv_bin(lambda s, kk: s * kk, step, k))
         for n, v in zip(iter_names, vals):
             inner[n] = v
+        tr.iterations.append(k)
         r = tr.trace_region(reg.ops, inner)
+        tr.iterations.pop()
         if isinstance(r, _Yield):
             vals = list(r.values)
             _lx_bind_carried(tr, iter_names, vals)

@@ -1,4 +1,6 @@
 """Products with few tiles: 128 x 64 / 128 x 128 tiles, K in ranges that a cluster adds up."""
+import re
+
 import numpy as np
 import pytest
 
@@ -73,3 +75,53 @@ def test_a_ranks_part_adds_up_like_the_whole():
         part = Session(R.PlanOnlyDevice(), func, t, {}, arena_ptr=0, shard=(rank, 4)).plan.statements[0].args
         assert part.M == 64 and (part.tile_n, part.split_k) == (whole.tile_n, whole.split_k)
     assert whole.split_k == 4
+
+
+ADD_THEN_MUL = """
+    %q_c = ktdp.get_compute_tile_id : index
+    %q_blk = arith.constant 128 : index
+    %q_c3 = arith.constant 3 : index
+    %q_c4 = arith.constant 4 : index
+    %q_half = arith.constant 512 : index
+    %q_off = arith.muli %q_c, %q_blk : index
+    %q_c7 = arith.addi %q_c, %q_c3 : index
+    %q_far = arith.divui %q_c7, %q_c4 : index
+    %q_skip = arith.muli %q_far, %q_half : index
+    %q_from = arith.addi %q_off, %q_skip : index
+""" + "".join(f"""    %q_{n}v = ktdp.construct_memory_view %{n}_ptr, sizes: [1024], strides: [1] {{
+      coordinate_set = affine_set<(d0) : (d0 >= 0, -d0 + 1023 >= 0)>, memory_space = #ktdp.memory_space<global>
+    }} : memref<1024xf16>
+""" for n in "xoz") + "".join(f"""    %q_{n}t = ktdp.construct_access_tile %q_{v}v[%q_{off}] {{
+      access_tile_set = affine_set<(d0) : (d0 >= 0, -d0 + 127 >= 0)>, access_tile_order = affine_map<(d0) -> (d0)>
+    }} : memref<1024xf16> -> !ktdp.access_tile<128xindex>
+""" for n, v, off in (("x", "x", "off"), ("o", "o", "off"), ("r", "o", "from"), ("z", "z", "off"))) + """
+    %q_x = ktdp.load %q_xt : !ktdp.access_tile<128xindex> -> tensor<128xf16>
+    %q_s = arith.addf %q_x, %q_x : tensor<128xf16>
+    ktdp.store %q_s, %q_ot : tensor<128xf16>, !ktdp.access_tile<128xindex>
+    %q_r = ktdp.load %q_rt : !ktdp.access_tile<128xindex> -> tensor<128xf16>
+    %q_m = arith.mulf %q_r, %q_x : tensor<128xf16>
+    ktdp.store %q_m, %q_zt : tensor<128xf16>, !ktdp.access_tile<128xindex>
+"""
+
+
+def test_statements_of_a_rank_follow_those_of_the_same_store():
+    """Core 0 multiplies what it has just added up, the others old values: the two stores are two launches in the whole
+    grid and one on the ranks without core 0.  The products behind them keep the ranges of K of their own counterparts."""
+    def body(src, name):
+        text = src[src.index("\n", src.index("func.func")) + 1:src.index("    return")]
+        return re.sub(r"%(\w+)", lambda m: f"%{name}_{m.group(1)}", text)
+    src = ('module {\n  func.func @k(%x_ptr: index, %o_ptr: index, %z_ptr: index, %m_a_ptr: index, %m_b_ptr: index, %m_c_ptr: index, '
+           '%n_a_ptr: index, %n_b_ptr: index, %n_c_ptr: index) attributes {grid = [4, 1]} {' + ADD_THEN_MUL +
+           body(K.tiled_matmul(256, 64, 4096, 64, 64, 64, 4, True), "m") + body(K.tiled_matmul(256, 64, 128, 64, 64, 64, 4, True), "n") +
+           "    return\n  }\n}\n")
+    f16 = np.dtype(np.float16)
+    t = [(k, (1024,), f16) for k in ("x_ptr", "o_ptr", "z_ptr")]
+    t += [(f"{n}_{k}_ptr", s, f16) for n, kd in (("m", 4096), ("n", 128)) for k, s in (("a", (256, kd)), ("b", (kd, 64)), ("c", (256, 64)))]
+    func = KTIRParser().parse_module(src).get_function("k")
+    kinds = lambda s: [x.kind for x in s.plan.statements]                                             # noqa: E731
+    cuts = lambda s: [(x.args.K, x.args.split_k) for x in s.plan.statements if x.kind == "gemm_f16"]  # noqa: E731
+    whole = Session(R.PlanOnlyDevice(), func, t, {}, arena_ptr=0)
+    assert kinds(whole) == ["ew_stream", "ew_stream", "gemm_f16", "gemm_f16"] and cuts(whole) == [(4096, 4), (128, 1)]
+    for rank in range(4):
+        part = Session(R.PlanOnlyDevice(), func, t, {}, arena_ptr=0, shard=(rank, 4))
+        assert kinds(part) == kinds(whole)[0 if rank == 0 else 1:] and cuts(part) == cuts(whole)
