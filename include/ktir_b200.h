@@ -471,9 +471,11 @@ typedef struct {
        then per K/V head, piece and row 32 times 24 bytes.  scratch_heads: the K/V heads that the scratch is laid out for,
        the same for every launch that shares it (a launch over some of the heads, say) and no less than the launch has;
        0: those of this launch.  Launches that share scratch must be ordered.  0 / NULL: one CTA per query head, as for
-       any number of rows. */
+       any number of rows.  steps: 64-position steps that the pieces are cut from, 0: those that the launch's rows see (a
+       launch over some rows of a statement names the whole's, so that a row is summed in the same pieces). */
     int32_t splits, scratch_heads;
     void* dev_scratch;
+    int32_t steps, reserved;
 } ktb_attn_args;
 int ktb_launch_attention_fwd(ktb_ctx* ctx, const ktb_attn_args* args);
 

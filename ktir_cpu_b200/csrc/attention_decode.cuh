@@ -364,7 +364,10 @@ static int launch_attn_decode(ktb_ctx* ctx, const ktb_attn_args& a, const CUtens
     const int kv_heads = a.heads / group, rows = a.seq_q * group;
     int64_t seen = (int64_t)a.num_tiles * a.page;                    // positions that some row sees
     if (a.causal && (int64_t)a.seq_q + a.causal_delta < seen) seen = (int64_t)a.seq_q + a.causal_delta;
-    const int steps = (int)((seen + AD_ROWS - 1) / AD_ROWS);
+    const int64_t least = (seen + AD_ROWS - 1) / AD_ROWS, most = ((int64_t)a.num_tiles * a.page + AD_ROWS - 1) / AD_ROWS;
+    if (a.steps != 0 && (a.steps < least || a.steps > most))
+        return ktb_fail(ctx, KTB_E_ARG, "attention_fwd", "steps must cover the positions that the rows see, within the context");
+    const int steps = a.steps ? a.steps : (int)least;
     // the largest cluster that the pieces fill
     int cluster = 1;
     while (cluster < AD_CLUSTER && a.splits % (cluster * 2) == 0) cluster *= 2;

@@ -300,17 +300,13 @@ class AttentionStatement(Statement):
         kv_heads, q_rows = heads // grp, seq_q * grp
         if q_rows <= DECODE_ROWS and heads % grp == 0:
             seen = min(T * tn, seq_q + delta) if m["causal"] else T * tn
-            a.splits = max(1, min(-(-seen // 64), DECODE_CTAS // kv_heads))
-            if a.splits > 4:                      # whole clusters of four pieces; below that of 2^n
-                a.splits -= a.splits % 4
+            steps = -(-seen // 64)
+            splits = max(1, min(steps, DECODE_CTAS // kv_heads))
+            if splits > 4:                        # whole clusters of four pieces; below that of 2^n
+                splits -= splits % 4
             else:
-                a.splits = 1 << (a.splits.bit_length() - 1)
-            a.scratch_heads = kv_heads            # (parts of the statement keep it: their counters are the whole's)
-            counters = (kv_heads * 8 * 4 + 255) // 256 * 256
-            a.dev_scratch = dev.alloc(counters + kv_heads * a.splits * q_rows * 32 * 24)
-            dev.memset(a.dev_scratch, 0, counters)
-            dev.sync()                            # (the context may be moved to another stream before the first run)
-            self.device_arrays = [a.dev_scratch]
+                splits = 1 << (splits.bit_length() - 1)
+            self._cut(dev, splits, steps)
         vis = np.minimum(T * tn, np.arange(seq_q) + 1 + delta) if m["causal"] else np.full(seq_q, T * tn)
         self.flops = int(4 * heads * hd * vis.sum())
         self._bytes = hd * 2 * (2 * heads * seq_q + 2 * ngrp * min(T, n_pages) * tn)
@@ -323,6 +319,27 @@ class AttentionStatement(Statement):
                     Footprint(os_, os_ + hd * 2, np.repeat(neg, nr), np.repeat(neg, nr), True, stmt_id)]
         for al in (kalloc, valloc, bt_alloc):
             self.fps.append(Footprint(np.array([al.byte_lo]), np.array([al.byte_hi]), neg, neg, False, stmt_id))
+
+    def _cut(self, dev, splits: int, steps: int):
+        """Cut the ``steps`` of the context into ``splits`` pieces, with scratch to merge them in (0: no pieces)."""
+        a = self.args
+        for ptr in self.device_arrays:
+            dev.free(ptr)
+        self.device_arrays, a.dev_scratch = [], None
+        a.splits, a.steps, a.scratch_heads = splits, steps, 0
+        if splits:
+            a.scratch_heads = kv_heads = a.heads // a.kv_group   # (parts keep it: their counters are the whole's)
+            counters = (kv_heads * 8 * 4 + 255) // 256 * 256
+            a.dev_scratch = dev.alloc(counters + kv_heads * splits * a.seq_q * a.kv_group * 32 * 24)
+            dev.memset(a.dev_scratch, 0, counters)
+            dev.sync()                            # (the context may be moved to another stream before the first run)
+            self.device_arrays = [a.dev_scratch]
+
+    def follow(self, whole: "AttentionStatement", dev):
+        """The pieces that the whole grid's rows are summed in, whatever heads and rows of it are here."""
+        a, w = self.args, whole.args
+        if (a.page, a.num_tiles, a.kv_group) == (w.page, w.num_tiles, w.kv_group) and (a.splits, a.steps) != (w.splits, w.steps):
+            self._cut(dev, w.splits, w.steps)
 
     def launch(self, dev, arena_ptr):
         self.args.arena = arena_ptr

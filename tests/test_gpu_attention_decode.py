@@ -128,3 +128,58 @@ def test_counters_are_zero_before_planning_returns():
             [(k, v.shape, v.dtype) for k, v in kw.items() if isinstance(v, np.ndarray)],
             {k: v for k, v in kw.items() if not isinstance(v, np.ndarray)}, arena_ptr=0)
     assert calls == [("memset", 0, 256), ("sync",)]
+
+
+# (tokens, positions before, query heads, K/V heads, rows per tile, ranks): heads dealt out; tokens dealt out, the context of
+# the first ones a step shorter; more rows in the whole than the pieces take, fewer on a rank
+SHARDS = [(1, 2100, 64, 8, 1, 2), (1, 2100, 64, 8, 1, 8), (4, 62, 4, 1, 1, 4), (4, 1021, 4, 1, 1, 2), (40, 500, 1, 1, 8, 5), (2, 900, 6, 3, 1, 3)]
+
+
+def _shard_case(tokens, before, heads, kv_heads, q):
+    src, kw = _case(tokens, before, heads, kv_heads, 64)
+    return K.paged_attention(tokens, before + tokens, heads, kv_heads, 128, 64, q), kw
+
+
+@pytest.mark.parametrize("tokens,before,heads,kv_heads,q,world", SHARDS)
+def test_a_rank_cuts_the_context_as_the_whole_grid(tokens, before, heads, kv_heads, q, world):
+    src, kw = _shard_case(tokens, before, heads, kv_heads, q)
+    func = KTIRParser().parse_module(src).get_function("paged_attention_kernel")
+
+    class Device(R.PlanOnlyDevice):
+        held = []
+
+        def alloc(self, nbytes):
+            self.held.append(nbytes)
+            return nbytes
+
+        def free(self, ptr):
+            self.held.remove(ptr)
+
+    def plan(shard, dev):
+        s = Session(dev, func, [(k, v.shape, v.dtype) for k, v in kw.items() if isinstance(v, np.ndarray)],
+                    {k: v for k, v in kw.items() if not isinstance(v, np.ndarray)}, arena_ptr=0, shard=shard)
+        st, = s.plan.statements
+        assert st.kind == "attention_fwd"
+        return st.args
+    whole = plan(None, R.PlanOnlyDevice())
+    for rank in range(world):
+        dev = Device()
+        dev.held = []
+        a = plan((rank, world), dev)
+        assert a.heads * a.seq_q * world == heads * tokens and (a.splits, a.steps) == (whole.splits, whole.steps)
+        n = a.heads // a.kv_group
+        assert dev.held == ([(n * 32 + 255) // 256 * 256 + n * a.splits * a.seq_q * a.kv_group * 768] if a.splits else [])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tokens,before,heads,kv_heads,q,world", SHARDS)
+def test_shards_give_the_bits_of_the_whole(tokens, before, heads, kv_heads, q, world, build_lib):
+    from test_gpu_parity import _sharded_on_one_gpu
+    src, kw = _shard_case(tokens, before, heads, kv_heads, q)
+    gpu = KTIRInterpreter()
+    gpu.load(src)
+    full = gpu.execute_function("paged_attention_kernel", **kw)["output_ptr"]
+    gpu.close()
+    got, covered = _sharded_on_one_gpu(src, "paged_attention_kernel", kw, world, "output_ptr")
+    np.testing.assert_array_equal(got.view(np.uint16), full.view(np.uint16))
+    assert covered == full.nbytes
