@@ -81,23 +81,36 @@ def match_matmul_loop(value: Node):
 SMS = 148                                        # of the B200
 
 
+CLUSTERS4 = 33                                   # of four CTAs with a whole SM's shared memory each, resident at once
+
+
 def few_tiles(M: int, N: int, K: int):
     """(tile_n, split_k) for a product that gives at most half of the CTA pairs a 256 x 256 tile, (0, 0) for the others.
 
     Tiles of 128 x 64 while they are no more than the SMs, and K in as many ranges, up to four, as still leave one CTA per
     SM and four steps of 64 each: f16 [512, 512, 4096] 12.4 us against 26.4 on pairs, [1024, 1024, 1024] 10.3 against
-    12.4, with two CTAs to an SM 16.5.  More tiles than that are 128 x 128 where K is long ([1536, 1536, 2048] 16.5 against
-    18.3) and left to the pairs where it is short ([848, 1408, 352] 8.2 against 12.3 on tiles of 64).  Where the pairs are
-    more than half busy they win: [2048, 2048, 512] 10.3 us against 16.8."""
+    12.4, with two CTAs to an SM 16.5.  Four ranges only while all clusters of four are resident at once: 36 of them
+    ([384, 768, 1280]) took 16.4 us, the 256-column tiles 11.4.  Two ranges from nine steps on ([64, 128, 512] 8.3 with two).
+    More tiles than that are 128 x 128 where K is long ([1536, 1536, 2048] 16.5 against 18.3) and left to the pairs where
+    it is short ([848, 1408, 352] 8.2 against 12.3 on tiles of 64).  Where the pairs are more than half busy they win:
+    [2048, 2048, 512] 10.3 us against 16.8.  Where the launcher would not use pairs but one CTA per 128 rows, that is the
+    better one for more than 64 rows up to 14 steps ([1024, 192, 384] 6.5 us against 8.2, [608, 128, 832] 8.3 against 9.3,
+    [640, 1024, 256] 6.2 against 7.2; from 15 steps on 10.3 against 9.3), and for many tiles below K = 2048 ([896, 2048,
+    1024] 10.3 against 11.7)."""
     cdiv = lambda x, y: -(-x // y)               # noqa: E731
     if cdiv(M, 256) * cdiv(N, 256) > SMS // 4:
         return 0, 0
-    tile_n = 64 if cdiv(M, 128) * cdiv(N, 64) <= SMS else 128
-    tiles = cdiv(M, 128) * cdiv(N, tile_n)
-    if tiles > SMS or (tile_n == 128 and K < 1024):
+    steps, row_tiles = cdiv(K, 64), cdiv(M, 128)
+    # (the launcher's choice of kernel)
+    pairs = (N % 256 == 0 or N >= 1024) and row_tiles >= 2 and (row_tiles % 2 == 0 or row_tiles >= 9)
+    if not pairs and M > 64 and steps < 15:
+        return 0, 0
+    tile_n = 64 if row_tiles * cdiv(N, 64) <= SMS else 128
+    tiles = row_tiles * cdiv(N, tile_n)
+    if tiles > SMS or (tile_n == 128 and K < (1024 if pairs else 2048)):
         return 0, 0
     split = 4
-    while split > 1 and (tiles * split > SMS or cdiv(K, 64) < 4 * split):
+    while split > 1 and (tiles > (CLUSTERS4 if split == 4 else SMS // split) or steps < 4 * split + (split == 2)):
         split //= 2
     return tile_n, split
 

@@ -121,7 +121,18 @@ def test_statements_of_a_rank_follow_those_of_the_same_store():
     kinds = lambda s: [x.kind for x in s.plan.statements]                                             # noqa: E731
     cuts = lambda s: [(x.args.K, x.args.split_k) for x in s.plan.statements if x.kind == "gemm_f16"]  # noqa: E731
     whole = Session(R.PlanOnlyDevice(), func, t, {}, arena_ptr=0)
-    assert kinds(whole) == ["ew_stream", "ew_stream", "gemm_f16", "gemm_f16"] and cuts(whole) == [(4096, 4), (128, 1)]
+    assert kinds(whole) == ["ew_stream", "ew_stream", "gemm_f16", "gemm_f16"] and cuts(whole) == [(4096, 4), (128, 0)]
     for rank in range(4):
         part = Session(R.PlanOnlyDevice(), func, t, {}, arena_ptr=0, shard=(rank, 4))
         assert kinds(part) == kinds(whole)[0 if rank == 0 else 1:] and cuts(part) == cuts(whole)
+
+
+@pytest.mark.parametrize("shape,plan", [
+    # the one-CTA kernel on 128 rows takes them up to 14 steps, and many tiles up to K = 2048 ...
+    ((1024, 192, 384), (0, 0)), ((608, 128, 832), (0, 0)), ((640, 1024, 256), (0, 0)), ((65, 512, 896), (0, 0)), ((896, 2048, 1024), (0, 0)),
+    # ... not beyond, nor up to 64 rows, nor where pairs would run
+    ((608, 128, 897), (64, 2)), ((64, 512, 448), (64, 1)), ((256, 512, 192), (64, 1)), ((896, 2048, 2048), (128, 1)), ((1152, 1408, 1024), (128, 1)),
+    # 33 clusters of four are resident at once; two ranges from nine steps on
+    ((384, 704, 1280), (64, 4)), ((384, 768, 1280), (64, 2)), ((1152, 256, 4096), (64, 2)), ((64, 128, 512), (64, 1)), ((64, 128, 576), (64, 2))])
+def test_products_that_the_other_kernels_are_faster_for(shape, plan):
+    assert few_tiles(*shape) == plan
