@@ -619,8 +619,8 @@ extern "C" int ktb_launch_attention_fwd(ktb_ctx* ctx, const ktb_attn_args* args)
             return ktb_fail(ctx, KTB_E_CUDA, "attention_fwd", "cuTensorMapEncodeTiled(Q) failed");
     }
     const int kvg = a.kv_group > 1 ? a.kv_group : 1;
-    // Up to 32 query rows per K/V head, and scratch to merge pieces of the context in: the decode kernel.
-    // (The line: 32 tokens of 32 heads over 544 positions cost 12.4 us either way, 16 over 2064 14.4 against 28.7.)
+    // Up to 32 query rows per K/V head, and pieces asked for with scratch to merge them in: the decode kernel.  (Where it is
+    // the faster one: decode_pieces in lower_attn.py, which chooses the pieces.)
     const bool decode = a.splits > 0 && a.dev_scratch && a.heads % kvg == 0 && (int64_t)a.seq_q * kvg <= AD_MAX_ROWS;
     if (decode && a.scratch_heads != 0 && a.scratch_heads < a.heads / kvg)
         return ktb_fail(ctx, KTB_E_ARG, "attention_fwd", "scratch laid out for fewer K/V heads than the launch has");

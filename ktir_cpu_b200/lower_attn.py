@@ -175,8 +175,50 @@ def match_attention(value: Node):
 
 
 # Query rows that share a K/V head, up to which the context is cut into pieces and spread over the SMs, and the CTAs that
-# makes (one per SM of the B200).
-DECODE_ROWS, DECODE_CTAS = 32, 148
+# makes: one per SM of the B200; in clusters of four no more than are resident at once (33 clusters).
+DECODE_ROWS, DECODE_CTAS, DECODE_CTAS4 = 32, 148, 132
+
+
+def decode_pieces(steps: int, page: int, rows: int, heads: int, kv_heads: int) -> int:
+    """Pieces that a context of ``steps`` 64-position steps is cut into for ``rows`` query rows per K/V head; 0: one CTA per
+    query head and no pieces.
+
+    While the query heads are one wave, one CTA for each is faster where a merge costs more than the steps it saves.  From
+    17 rows on (a second tile of 16) up to three steps (4 tokens, 32 / 4 heads, 128 positions 8.3 us against 11.5); with
+    pages above 32 rows (fewer waits per step) four for more than 18 rows (256 positions 9.3 against 10.3), six or seven
+    where four pieces per head are nearly all SMs (8 tokens, 128 / 32 heads, 384 positions 10.4 against 11.3), and three for
+    two waves (256 heads, 128 positions 10.3 against 11.3).  With two or three pieces per head up to twelve steps (32 tokens,
+    36 heads, 512 positions 12.4 against 14.5), five in pages of 32; with one always (75 heads, 5000 positions 57 against
+    68), seven steps in pages of 32.  From 10 rows on up to four steps with less than four pieces.
+    Of the rest, 10 rows and more take two or three steps in one piece (16 tokens, 4 heads, 128 positions in pages of 32:
+    9.2 us in two, 8.3 in one).  A second cluster per head pays from 12 steps on for more than 16 rows (512 positions 14.4
+    us in 8 pieces, 11.2 in 4).  36 clusters of four (18 heads in 8 pieces) took two waves: 17 us for 16 rows and 640
+    positions, 13 on the other kernel."""
+    if rows > DECODE_ROWS:
+        return 0
+    n = max(1, min(steps, DECODE_CTAS // kv_heads))
+    if n >= 4:
+        n = min(n, DECODE_CTAS4 // kv_heads)
+    spread = DECODE_CTAS4 // kv_heads >= 4               # four pieces per head at once
+    if heads <= DECODE_CTAS:
+        if rows > 16:
+            if spread:
+                most = 3 if page == 32 or rows <= 18 else 4 if kv_heads <= 18 else 7 if page == 64 else 6
+            elif DECODE_CTAS // kv_heads > 1:
+                most = 5 if page == 32 else 12
+            else:
+                most = 7 if page == 32 else steps
+            if steps <= most:
+                return 0
+        elif rows > 9 and not spread and page > 32 and steps <= 4:
+            return 0
+    elif rows > 16 and page > 32 and 1 < steps <= 3 and heads <= 2 * DECODE_CTAS:
+        return 0
+    if rows > 9 and steps <= 3:
+        return 1
+    if rows > 16 and steps < 12:
+        n = min(n, 4)
+    return n - n % 4 if n > 4 else 1 << (n.bit_length() - 1)      # whole clusters of four; below that of 2^n
 
 
 class AttentionStatement(Statement):
@@ -298,14 +340,10 @@ class AttentionStatement(Statement):
         a.scale, a.m_init, a.l_init = m["scale"], m["m_init"], m["l_init"]
         self.device_arrays = []
         kv_heads, q_rows = heads // grp, seq_q * grp
-        if q_rows <= DECODE_ROWS and heads % grp == 0:
-            seen = min(T * tn, seq_q + delta) if m["causal"] else T * tn
-            steps = -(-seen // 64)
-            splits = max(1, min(steps, DECODE_CTAS // kv_heads))
-            if splits > 4:                        # whole clusters of four pieces; below that of 2^n
-                splits -= splits % 4
-            else:
-                splits = 1 << (splits.bit_length() - 1)
+        seen = min(T * tn, seq_q + delta) if m["causal"] else T * tn
+        steps = -(-seen // 64)
+        splits = decode_pieces(steps, tn, q_rows, heads, kv_heads)
+        if splits:
             self._cut(dev, splits, steps)
         vis = np.minimum(T * tn, np.arange(seq_q) + 1 + delta) if m["causal"] else np.full(seq_q, T * tn)
         self.flops = int(4 * heads * hd * vis.sum())

@@ -7,6 +7,7 @@ import pytest
 
 from ktir_cpu_b200 import KTIRInterpreter, kernels as K, runtime as R
 from ktir_cpu_b200.interpreter import Session
+from ktir_cpu_b200.lower_attn import decode_pieces
 from ktir_cpu_b200.parser import KTIRParser
 from oracle.numpy_interp import OracleInterpreter
 
@@ -76,7 +77,7 @@ def test_pieces_fill_clusters_and_no_more_than_the_context(tokens, before, heads
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("kv_heads,group", [(17, 1), (18, 2), (8, 4), (32, 1)])
+@pytest.mark.parametrize("kv_heads,group", [(17, 1), (18, 2), (32, 1), (8, 4)])
 def test_whole_and_parts_share_the_scratch(kv_heads, group, build_lib):
     """Eight or more pieces (two clusters per head and slice, so the counters in scratch are used): launches over all
     heads, over parts of them and over all again, on one scratch, give the same bits, those of the oracle's bar."""
@@ -85,8 +86,10 @@ def test_whole_and_parts_share_the_scratch(kv_heads, group, build_lib):
     gpu.load(src)
     sess, _ = gpu.session("paged_attention_kernel", **kw)
     st, = sess.plan.statements
+    if kv_heads in (17, 18):             # (the planner would take four)
+        st._cut(gpu.device, 8, st.args.steps)
     parts = [c.launch for c in st.split(st.bytes_moved() // 4)]
-    assert len(parts) == 4 and (st.args.splits >= 8 or kv_heads == 32)
+    assert len(parts) == 4 and st.args.splits == (4 if kv_heads == 32 else 8 if kv_heads in (17, 18) else 16)
     for k, v in kw.items():
         if isinstance(v, np.ndarray):
             sess.upload(k, v)
@@ -183,3 +186,20 @@ def test_shards_give_the_bits_of_the_whole(tokens, before, heads, kv_heads, q, w
     got, covered = _sharded_on_one_gpu(src, "paged_attention_kernel", kw, world, "output_ptr")
     np.testing.assert_array_equal(got.view(np.uint16), full.view(np.uint16))
     assert covered == full.nbytes
+
+
+@pytest.mark.parametrize("steps,page,rows,heads,kv_heads,pieces", [
+    # a second tile of rows, query heads in one wave (two with pages above 32): few steps stay with one CTA per query head
+    (1, 64, 32, 32, 4, 0), (2, 32, 32, 32, 4, 0), (3, 32, 17, 4, 4, 0), (4, 32, 32, 32, 4, 4), (4, 64, 24, 32, 4, 0), (4, 64, 18, 8, 4, 4),
+    (5, 64, 32, 32, 4, 4), (7, 64, 32, 128, 32, 0), (8, 64, 32, 128, 32, 4), (6, 128, 32, 128, 32, 0), (7, 128, 32, 128, 32, 4), (6, 32, 32, 128, 32, 4), (2, 64, 32, 256, 32, 0), (2, 32, 32, 256, 32, 1),
+    (1, 64, 32, 256, 32, 1), (2, 64, 32, 1024, 128, 1), (4, 64, 32, 256, 32, 4),
+    # less than four pieces per head
+    (12, 64, 32, 36, 36, 0), (13, 64, 32, 36, 36, 2), (99, 64, 17, 75, 75, 0), (99, 64, 16, 75, 75, 1), (7, 32, 17, 75, 75, 0), (8, 32, 17, 75, 75, 1), (5, 32, 32, 36, 36, 0), (6, 32, 32, 36, 36, 2), (4, 64, 10, 36, 36, 0), (4, 32, 10, 36, 36, 2),
+    (4, 64, 9, 36, 36, 2), (12, 64, 32, 288, 36, 2),
+    # 10 to 16 rows: two or three steps in one piece
+    (2, 32, 16, 4, 4, 1), (3, 128, 10, 4, 4, 1), (3, 64, 9, 4, 4, 2), (4, 64, 16, 4, 4, 4),
+    # a second cluster per head from 12 steps on, for up to 16 rows at once; no more clusters than are resident
+    (8, 64, 32, 32, 4, 4), (12, 64, 32, 32, 4, 12), (8, 64, 16, 16, 4, 8), (16, 64, 8, 144, 18, 4), (200, 64, 8, 136, 17, 4), (200, 64, 8, 128, 16, 8),
+    (200, 64, 8, 32, 4, 32), (200, 64, 8, 264, 33, 4), (200, 64, 8, 272, 34, 2), (200, 64, 8, 592, 74, 2), (200, 64, 8, 600, 75, 1), (200, 64, 33, 33, 1, 0)])
+def test_pieces_of_a_context(steps, page, rows, heads, kv_heads, pieces):
+    assert decode_pieces(steps, page, rows, heads, kv_heads) == pieces
