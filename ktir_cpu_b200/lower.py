@@ -382,8 +382,11 @@ class EwStatement(Statement):
         vec = (self._cols % 8 == 0) and bool((table % 8 == 0).all()) and \
             all(c[1] % 8 == 0 or self._rows == 1 for c in self._cols_of)
         # One add / sub / mul / div / max / min / copy has a kernel compiled for it, which runs at the copy rate (f32
-        # add of 2^24 elements 33.4 us for 201 MB); all else goes to the kernel that decodes its ops (exp of as many
-        # 34.9 us for 134 MB).
+        # add of 2^24 elements 33.4 us for 201 MB).  The same launcher takes one store of any other program where it is
+        # faster than the kernel that decodes its ops for several stores: two inputs and more, f32 among them, on
+        # boundaries (x * y + y, f32[2^24]: 57.4 us against 72.0), and programs of several ops over a few elements that
+        # start anywhere, one to a thread (three ops, f32, blocks of 333: 63936 elements 4.2 us against 6.2, 127872 6.2
+        # either way, 255744 8.3 against 6.2).  All else goes to the latter (exp, f32[2^24]: 34.9 us for 134 MB).
         p = self.program = self._programs[0]
         special = p.n_ops == 0 and p.result_reg == 0 and n_in == 1
         if p.n_ops == 1:
@@ -391,7 +394,9 @@ class EwStatement(Statement):
             code = R.VM_OPS[op.opcode & 0xff] if (op.opcode & 0xff) < len(R.VM_OPS) else ""
             special = op.a == 0 and op.dst == p.result_reg and \
                 (code == "MOV" or (n_in == 2 and op.b == 1 and code in ("ADD", "SUB", "MUL", "DIV", "MAX", "MIN")))
-        self._multi = len(self._programs) > 1 or self._extra or not special
+        wide = vec and n_in >= 2 and any(c[2] != "f16" for c in self._cols_of[:n_in])
+        short = not vec and p.n_ops >= 2 and table.shape[0] * self._rows * self._cols < 1 << 17
+        self._multi = len(self._programs) > 1 or self._extra or not (special or wide or short)
         self.symbol = "ktb_launch_ew_multi" if self._multi else "ktb_launch_ew_stream"
         self.args = a = R.EwMultiArgs() if self._multi else R.EwArgs()
         a.n_items, a.rows, a.cols = table.shape[0], self._rows, self._cols

@@ -92,3 +92,41 @@ def test_which_stores_join():
     one, = _plan(K.elementwise_suite(["add"], 4096, 128, 4, "f32"), "elementwise_kernel",
                  [(k, (4096,), np.dtype(np.float32)) for k in ("x_ptr", "y_ptr", "out_add_ptr")])
     assert one.symbol == "ktb_launch_ew_stream"
+
+
+def _chain(n, block, dtype, ops):
+    """x (op) y (op) y ..., one store."""
+    src, prev, text = K.vector_add(n, block, 4, dtype), "%x", ""
+    for i, op in enumerate(ops):
+        text += f"%q{i} = math.{op} {prev}" if op in ("exp", "sqrt") else f"%q{i} = arith.{op} {prev}, %y"
+        text, prev = text + f" : tensor<{block}x{dtype}>\n    ", f"%q{i}"
+    at = src.index("%output = arith.addf")
+    return src[:at] + text.rstrip() + src[src.index("\n", at):].replace("ktdp.store %output,", f"ktdp.store {prev},")
+
+
+# (elements, block, dtype, ops) and whether the kernel for several stores takes it
+ROUTES = [(8192, 128, "f32", ["mulf", "addf"], False), (8192, 128, "f32", ["minnumf"], False), (8192, 128, "f32", ["exp"], True),
+          (8192, 128, "f16", ["mulf", "addf"], True), (8192, 128, "f16", ["mulf"], False), (333 * 12, 333, "f16", ["mulf", "exp", "divf"], False),
+          (333 * 12, 333, "f32", ["mulf", "sqrt"], False), (333 * 12, 333, "f32", ["exp"], True), (1025 * 128, 1025, "f16", ["mulf", "addf"], True)]
+
+
+@pytest.mark.parametrize("n,block,dtype,ops,multi", ROUTES)
+def test_which_kernel_takes_one_store(n, block, dtype, ops, multi):
+    t = [(k, (n,), np.dtype(np.float16 if dtype == "f16" else np.float32)) for k in ("x_ptr", "y_ptr", "output_ptr")]
+    func = KTIRParser().parse_module(_chain(n, block, dtype, ops)).get_function("add_kernel")
+    st, = Session(R.PlanOnlyDevice(), func, t, dict(BLOCK_SIZE=block), arena_ptr=0).plan.statements
+    assert st.kind == "ew_stream" and st.symbol == ("ktb_launch_ew_multi" if multi else "ktb_launch_ew_stream")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,block,dtype,ops,multi", ROUTES)
+def test_one_store_gives_the_bits_of_the_step_by_step_path(n, block, dtype, ops, multi, build_lib):
+    a = _args([], n, dtype, None)
+    kw = dict(x_ptr=a["x_ptr"], y_ptr=a["y_ptr"], output_ptr=np.full_like(a["x_ptr"], 7), BLOCK_SIZE=block)
+    got = []
+    for fused in (True, False):
+        it = KTIRInterpreter(fused_kernels=fused)
+        it.load(_chain(n, block, dtype, ops))
+        got.append(it.execute_function("add_kernel", **kw)["output_ptr"].view(np.uint8))
+        it.close()
+    np.testing.assert_array_equal(got[0], got[1])
