@@ -874,9 +874,13 @@ extern "C" int ktb_launch_row_program(ktb_ctx* ctx, const ktb_rowprog_args* args
     // Rows of more than 512 elements, and few rows of any length, go to the kernel that parks the row in shared memory:
     // layer norm f16[2048, 8192] 28.9 us against 69.5 in registers, blocked f16[4096, 8 x 1024] 59.2 against 82.1,
     // [8192, 1024] 20.6 against 31.0, [256, 256] 6.2 against 9.8.  Many short rows stay in registers, several to a
-    // warp: [16384, 512] 30.3 against 34.2, [32768, 128] 20.2 against 41.0.
+    // warp: [16384, 512] 30.3 against 34.2, [32768, 128] 20.2 against 41.0, and so do more than 3 * 2^18 elements in short
+    // rows (rms norm [2016, 512] 6.2 against 8.3; [1536, 512] the same) and two short column blocks (f16[1024, 2 x 512] 9.1
+    // against 10.4, [256, 2 x 1024] 8.3 against 10.3).
     int rc_any;
-    if (matched && ((int64_t)(nm.blocked ? a.n_blocks : 1) * a.cols > 512 || total_rows <= 2048) &&
+    const int64_t elems = (int64_t)(nm.blocked ? a.n_blocks : 1) * a.cols;
+    const bool two_blocks = matched && nm.blocked && a.n_blocks == 2 && (elems <= 1024 || (elems <= 2048 && total_rows <= 512));
+    if (matched && !two_blocks && (elems > 512 || (total_rows <= 2048 && total_rows * elems <= (3 << 18))) &&
         rp_try_norm_any(ctx, a, nm, total_rows, &rc_any))
         return rc_any;
     if (matched && (nm.blocked || nm.r16)) {

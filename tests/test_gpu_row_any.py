@@ -114,3 +114,25 @@ def test_log_softmax_rows_of_any_length(rows, cols, cores, step, build_lib):
                                       dict(x_ptr=x, y_ptr=np.zeros_like(x)))
     assert kinds == ["row_program"] and symbols == ["ktb_launch_row_program_any"]
     np.testing.assert_allclose(got["y_ptr"].astype(np.float32), want["y_ptr"].astype(np.float32), rtol=2e-3, atol=2e-3)
+
+
+@pytest.mark.parametrize("rows,block", [(13, 512), (512, 1024), (513, 1024), (7, 8)])
+def test_two_column_blocks(rows, block, build_lib):
+    """Two short blocks stay on the kernel that holds the row in registers; both sides of its line."""
+    rng = np.random.default_rng(rows)
+    rc = (rows, 2 * block)
+    kw = dict(X=rng.standard_normal(rc).astype(np.float16), Y=np.zeros(rc, np.float16), W=rng.standard_normal(rc).astype(np.float16),
+              B=rng.standard_normal(rc).astype(np.float16), Mean=np.zeros(rows, np.float16), Rstd=np.zeros(rows, np.float16), N=rc[1],
+              eps=np.float16(1e-5), BLOCK_SIZE=block)
+    got, want, kinds, _ = _both(K.layernorm_blocked(*rc, block, 4), "_layer_norm_fwd_fused", kw)
+    assert kinds == ["row_program"]
+    _bits(got, want, ("Mean", "Rstd", "Y"))
+
+
+@pytest.mark.parametrize("rows", [1536, 1540])
+def test_many_short_rows(rows, build_lib):
+    rng = np.random.default_rng(rows)
+    kw = dict(x_ptr=rng.standard_normal((rows, 512)).astype(np.float16), y_ptr=np.zeros((rows, 512), np.float16), rstd_ptr=np.zeros(rows, np.float32))
+    got, want, kinds, _ = _both(K.rmsnorm_rows(rows, 512, 4, 1), "rmsnorm_kernel", kw)
+    assert kinds == ["row_program"]
+    _bits(got, want, ("y_ptr", "rstd_ptr"))
