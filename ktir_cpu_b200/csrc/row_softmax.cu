@@ -517,10 +517,10 @@ ktb_row_softmax_any_h_kernel(const ktb_softmax_args a, int T, int64_t total_rows
 }
 
 template <int NV>
-static int launch_softmax_any(ktb_ctx* ctx, const ktb_softmax_args& a, const rg_split& s, int64_t total_rows) {
+static int launch_softmax_any(ktb_ctx* ctx, const ktb_softmax_args& a, const rg_split& s, int64_t total_rows, bool packed) {
     const unsigned blocks = (unsigned)((total_rows + s.groups - 1) / s.groups), threads = s.threads * s.groups;
     const bool mn = a.max_is_maxnum != 0, r16 = a.f16_arith != 0;
-    if (a.in_dtype == KTB_F16 && a.out_dtype == KTB_F16 && !r16) {
+    if (packed) {
         if (mn) ktb_row_softmax_any_h_kernel<NV, true><<<blocks, threads, 0, ctx->stream>>>(a, s.threads, total_rows);
         else ktb_row_softmax_any_h_kernel<NV, false><<<blocks, threads, 0, ctx->stream>>>(a, s.threads, total_rows);
     } else if constexpr (NV <= 4) {
@@ -546,17 +546,19 @@ extern "C" int ktb_launch_row_softmax_any(ktb_ctx* ctx, const ktb_softmax_args* 
         return ktb_fail(ctx, KTB_E_UNSUPPORTED, "row_softmax_any", "dtype must be f16 or f32");
     const int64_t total_rows = a.n_items * (int64_t)a.rows_per_item;
     if (total_rows >= (1ll << 31)) return ktb_fail(ctx, KTB_E_UNSUPPORTED, "row_softmax_any", "more than 2^31 rows");
-    // packed halves: up to 8 chunks per thread (128 bytes in flight each), f32 values: up to 4
-    const bool packed = a.in_dtype == KTB_F16 && a.out_dtype == KTB_F16 && !a.f16_arith;
+    // packed halves: up to 8 chunks per thread (128 bytes in flight each), f32 values: up to 4.  The packed form takes the
+    // usual initial values only: its exponential flushes what lies below the normal numbers, which shows when the maximum
+    // starts far above every element, and the common factor that its quotient leaves out is no factor of an initial sum.
+    const bool packed = a.in_dtype == KTB_F16 && a.out_dtype == KTB_F16 && !a.f16_arith && a.max_init <= -65504.f && a.sum_init == 0.f;
     const rg_split s = rg_choose(a.cols, aligned, total_rows, ctx->sm_count, packed ? 8 : 4, packed ? 256 : 512);
     switch (s.nv) {
-        case 1: return launch_softmax_any<1>(ctx, a, s, total_rows);
-        case 2: return launch_softmax_any<2>(ctx, a, s, total_rows);
-        case 3: return launch_softmax_any<3>(ctx, a, s, total_rows);
-        case 4: return launch_softmax_any<4>(ctx, a, s, total_rows);
-        case 5: return launch_softmax_any<5>(ctx, a, s, total_rows);
-        case 6: return launch_softmax_any<6>(ctx, a, s, total_rows);
-        case 7: return launch_softmax_any<7>(ctx, a, s, total_rows);
-        default: return launch_softmax_any<8>(ctx, a, s, total_rows);
+        case 1: return launch_softmax_any<1>(ctx, a, s, total_rows, packed);
+        case 2: return launch_softmax_any<2>(ctx, a, s, total_rows, packed);
+        case 3: return launch_softmax_any<3>(ctx, a, s, total_rows, packed);
+        case 4: return launch_softmax_any<4>(ctx, a, s, total_rows, packed);
+        case 5: return launch_softmax_any<5>(ctx, a, s, total_rows, packed);
+        case 6: return launch_softmax_any<6>(ctx, a, s, total_rows, packed);
+        case 7: return launch_softmax_any<7>(ctx, a, s, total_rows, packed);
+        default: return launch_softmax_any<8>(ctx, a, s, total_rows, packed);
     }
 }

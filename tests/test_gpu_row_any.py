@@ -136,3 +136,24 @@ def test_many_short_rows(rows, build_lib):
     got, want, kinds, _ = _both(K.rmsnorm_rows(rows, 512, 4, 1), "rmsnorm_kernel", kw)
     assert kinds == ["row_program"]
     _bits(got, want, ("y_ptr", "rstd_ptr"))
+
+
+def _initial(src, max_init, sum_init):
+    """The softmax kernel with other initial values of its two reductions."""
+    for name, old, value in (("max_init", "ninf", max_init), ("sum_init", "zero", sum_init)):
+        assert src.count(f"%{name} = tensor.splat %{old} : ") == 1
+        src = src.replace(f"%{name} = tensor.splat %{old} : ", f"%{name}_v = arith.constant {value} : f32\n      %{name} = tensor.splat %{name}_v : ")
+    return src
+
+
+@pytest.mark.parametrize("cols", [250, 3000])
+@pytest.mark.parametrize("max_init,sum_init,low,high", [("0.0", "0.0", -96, -89), ("0.0", "0.0", -3, 3), ("-65504.0", "0.0", -3, 3), ("-3.0e38", "0.0", -3, 3),
+                                                        ("-3.0e38", "1.0", 59000, 60000), ("-3.0e38", "0.5", -3, 3)])
+def test_softmax_with_initial_values(cols, max_init, sum_init, low, high, build_lib):
+    """A maximum that starts above every element leaves weights, and a sum, below the normal numbers of f32 (spaced 2^-149:
+    2^-10 of the smallest sum here, 250 e^-96); a sum that starts at one is not scaled with the rest.  As f16, 2^-11."""
+    x = np.random.default_rng(cols).uniform(low, high, (8, cols)).astype(np.float16)
+    src = _initial(K.softmax_rows(8, cols, 4, 2, True), max_init, sum_init)
+    got, want, kinds, symbols = _both(src, "softmax_kernel", dict(output_ptr=np.zeros_like(x), input_ptr=x))
+    assert kinds == ["row_softmax"] and symbols == ["ktb_launch_row_softmax_any"]
+    np.testing.assert_allclose(got["output_ptr"].astype(np.float32), want["output_ptr"].astype(np.float32), rtol=2e-3, atol=2e-6)
