@@ -622,8 +622,8 @@ class SoftmaxStatement(Statement):
         if (gi.rows, gi.cols, len(gi.lead)) != (go.rows, go.cols, len(go.lead)):
             raise Unsupported("softmax input and output tiles differ in shape")
         cols = gi.cols
-        if cols > 16384:
-            raise Unsupported(f"fused softmax over rows of {cols} elements (16384 at most)")
+        if not 1 <= cols <= 16384:
+            raise Unsupported(f"fused softmax over rows of {cols} elements (1 to 16384)")
         sel, cores = _points(store)
         n_lead = len(gi.lead)
         table = np.empty((len(sel) * n_lead, 2), np.int64)

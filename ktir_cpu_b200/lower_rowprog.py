@@ -248,8 +248,8 @@ class RowProgramStatement(Statement):
         if not src_shape:
             raise Unsupported("reduction of a scalar")
         cols, full = int(src_shape[-1]), _prod(src_shape)
-        if cols > 16384:
-            raise Unsupported(f"row program over rows of {cols} elements (16384 at most)")
+        if not 1 <= cols <= 16384:
+            raise Unsupported(f"row program over rows of {cols} elements (1 to 16384)")
         aligned = True                                       # cleared below where a row starts off a boundary
         rows_total = full // cols
         per_row = _prod(tgt.shape) == rows_total and rows_total != full

@@ -246,3 +246,16 @@ def test_run_overlap_check_behind_the_absorption_of_per_row_results():
         s1 = rng.integers(0, 200, 7); e1 = s1 + rng.integers(1, 30, 7)
         want = bool(((s0[:, None] < e1[None, :]) & (s1[None, :] < e0[:, None])).any())
         assert _runs_overlap(s0, e0, s1, e1) == want
+
+
+@pytest.mark.parametrize("make,fn,names", [(lambda: K.softmax_rows(8, 30, 4, 1, True), "softmax_kernel", ("output_ptr", "input_ptr")),
+                                           (lambda: K.log_softmax_rows(8, 30, 4, 1), "log_softmax_kernel", ("x_ptr", "y_ptr"))])
+def test_rows_without_elements_are_planned_step_by_step(make, fn, names):
+    from ktir_cpu_b200.runtime import PlanOnlyDevice
+    src = make()
+    box = "(d0 >= 0, -d0 + 0 >= 0, d1 >= 0, -d1 + 29 >= 0)>"
+    assert src.count(box) >= 2
+    src = src.replace(box, "(d0 >= 0, -d0 + 0 >= 0, d1 >= 0, -d1 - 1 >= 0)>").replace("1x30x", "1x0x")
+    t = [(k, (8, 30), np.dtype(np.float16)) for k in names]
+    sess = Session(PlanOnlyDevice(), KTIRParser().parse_module(src).get_function(fn), t, {}, arena_ptr=0)
+    assert [s.kind for s in sess.plan.statements] == ["generic"]
