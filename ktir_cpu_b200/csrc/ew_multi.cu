@@ -347,6 +347,17 @@ __global__ void __launch_bounds__(256, 4) ktb_ew_multi_any_kernel(const __grid_c
     });
 }
 
+// Registers that an op reads, as bits.
+static uint32_t em_reads(const ktb_vm_op& op) {
+    const int code = op.opcode & 0xff;
+    if (code == KTB_VM_CONST) return 0;
+    uint32_t r = 1u << op.a;
+    if ((code >= KTB_VM_ADD && code <= KTB_VM_MINNUM) || code == KTB_VM_FMA || code == KTB_VM_CSEL) r |= 1u << op.b;
+    if (code == KTB_VM_FMA || code == KTB_VM_CSEL) r |= 1u << op.c;
+    if (code == KTB_VM_CSEL) r |= 1u << ((int)op.imm & 7);
+    return r;
+}
+
 extern "C" int ktb_launch_ew_multi(ktb_ctx* ctx, const ktb_ew_multi_args* args) {
     if (!ctx || !args) return KTB_E_ARG;
     const ktb_ew_multi_args& a = *args;
@@ -358,6 +369,7 @@ extern "C" int ktb_launch_ew_multi(ktb_ctx* ctx, const ktb_ew_multi_args* args) 
         if (p.n_in != a.n_in || p.n_ops < 0 || p.n_ops > KTB_VM_MAX_OPS || p.result_reg < 0 || p.result_reg >= KTB_VM_REGS ||
             (p.n_ops == 0 && p.result_reg >= a.n_in))
             return ktb_fail(ctx, KTB_E_ARG, "ew_multi", "bad program header");
+        uint32_t held = (1u << a.n_in) - 1;              // registers that hold a value: the inputs, then what has been written
         for (int i = 0; i < p.n_ops; ++i) {
             const ktb_vm_op& op = p.ops[i];
             const int code = op.opcode & 0xff;
@@ -366,6 +378,10 @@ extern "C" int ktb_launch_ew_multi(ktb_ctx* ctx, const ktb_ew_multi_args* args) 
                 return ktb_fail(ctx, KTB_E_ARG, "ew_multi", "bad program op");
             if (code == KTB_VM_CSEL && !(op.imm >= 0.f && op.imm < 8.f * 16))
                 return ktb_fail(ctx, KTB_E_ARG, "ew_multi", "bad comparison");
+            if (em_reads(op) & ~held) return ktb_fail(ctx, KTB_E_ARG, "ew_multi", "bad program op: it reads a register that holds nothing");
+            held |= 1u << op.dst;
+            // (a single op's result is stored from registers: nothing else can be asked for)
+            if (p.n_ops == 1 && p.result_reg != op.dst) return ktb_fail(ctx, KTB_E_ARG, "ew_multi", "bad program header: not the op's result");
             if (p.n_ops > 1) {
                 int top = op.dst > op.a ? op.dst : op.a;
                 top = top > op.b ? top : op.b;
@@ -374,6 +390,7 @@ extern "C" int ktb_launch_ew_multi(ktb_ctx* ctx, const ktb_ew_multi_args* args) 
                 if (top + 1 > regs) regs = top + 1;
             }
         }
+        if (!((held >> p.result_reg) & 1)) return ktb_fail(ctx, KTB_E_ARG, "ew_multi", "bad program header: a result that nothing wrote");
         if (p.n_ops > 1) {
             if (p.result_reg + 1 > regs) regs = p.result_reg + 1;
             if (a.n_in > regs) regs = a.n_in;
@@ -383,7 +400,8 @@ extern "C" int ktb_launch_ew_multi(ktb_ctx* ctx, const ktb_ew_multi_args* args) 
         if (a.dtype[k] != KTB_F16 && a.dtype[k] != KTB_F32)
             return ktb_fail(ctx, KTB_E_UNSUPPORTED, "ew_multi", "operand dtype must be f16 or f32");
     if (a.n_items <= 0 || a.rows <= 0 || a.cols <= 0) return KTB_OK;
-    const bool vec = a.vector_ok && a.cols % 8 == 0;
+    bool vec = a.vector_ok && a.cols % 8 == 0;
+    for (int k = 0; k < a.n_in + a.n_out; ++k) vec = vec && (a.rows == 1 || a.row_stride[k] % 8 == 0);
     const uint32_t per_row = vec ? a.cols / 8 : (a.cols + 14) / 8;
     const uint64_t per_item = (uint64_t)per_row * a.rows;
     if (per_item >= (1ull << 31) || a.n_items >= (1ll << 32)) return ktb_fail(ctx, KTB_E_UNSUPPORTED, "ew_multi", "tile too large");

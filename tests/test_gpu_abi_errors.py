@@ -257,3 +257,50 @@ def test_generic_step_launcher_refuses_unknown_kinds_and_extents(build_lib):
     a.kind, a.points, a.elems = R.G_KINDS["ew"], -1, 8
     _refused(dev, launch, a, E_ARG, "generic", "extents")
     dev.close()
+
+
+def test_elementwise_launcher_for_several_stores_refuses_bad_programs(build_lib):
+    rng = np.random.default_rng(8)
+    n = 1024
+    src = K.elementwise_suite(["add", "exp"], n, 128, 4, "f16", "olt")
+    names = ("out_add_ptr", "out_exp_ptr", "out_select_ptr", "out_ext_add_ptr")
+    kw = dict(x_ptr=rng.standard_normal(n).astype(np.float16), y_ptr=rng.standard_normal(n).astype(np.float16), **{k: np.zeros(n, np.float16) for k in names})
+    interp, sess = _session(src, "elementwise_kernel", kw)
+    dev, stmt = sess.dev, _only(sess, "ew_stream")
+    launch = dev.lib.ktb_launch_ew_multi
+    args = stmt.args
+    assert stmt.symbol == "ktb_launch_ew_multi" and (args.n_in, args.n_out) == (2, 4)
+    ops = [list(p.ops)[0].opcode & 0xff for p in list(args.program)[:4]]
+    add, exp, select = ops.index(R.VM["ADD"]), ops.index(R.VM["EXP"]), ops.index(R.VM_EXTRA["CSEL"])
+
+    def broken(change, code, *words):
+        a = _copy(args, sess.arena)
+        change(a)
+        _refused(dev, launch, a, code, "ew_multi", *words)
+
+    def setter(o, field, value):
+        return lambda a: setattr(a.program[o].ops[0], field, value)
+    broken(lambda a: setattr(a, "n_in", 0), E_ARG, "counts")
+    broken(lambda a: setattr(a, "n_out", R.EW_MAX_OUT + 1), E_ARG, "counts")
+    broken(lambda a: setattr(a.program[0], "n_ops", R.VM_MAX_OPS + 1), E_ARG, "program header")
+    broken(lambda a: setattr(a.program[add], "result_reg", 7), E_ARG, "program header")
+    broken(setter(add, "opcode", 0xff), E_ARG, "program op")
+    broken(setter(add, "dst", R.VM_REGS), E_ARG, "program op")
+    broken(setter(add, "b", 2), E_ARG, "holds nothing")
+    broken(setter(exp, "a", 5), E_ARG, "holds nothing")
+    broken(setter(select, "c", 3), E_ARG, "holds nothing")
+    broken(setter(select, "imm", 8.0 * R.CMP["olt"] + 6), E_ARG, "holds nothing")
+    broken(setter(select, "imm", 8.0 * 16), E_ARG, "comparison")
+
+    def longer(second):                              # two ops: the second reads what the first has not written
+        def change(a):
+            p = a.program[exp]
+            p.n_ops, p.result_reg = 2, second[1]
+            p.ops[1] = R.VmOp(*second)
+        return change
+    broken(longer((R.VM["ADD"], 4, 2, 5, 0, 0.0)), E_ARG, "holds nothing")
+    broken(longer((R.VM["FMA"], 4, 0, 1, 6, 0.0)), E_ARG, "holds nothing")
+    broken(lambda a: (longer((R.VM["NEG"], 4, 0, 0, 0, 0.0))(a), setattr(a.program[exp], "result_reg", 5)), E_ARG, "nothing wrote")
+    broken(lambda a: a.dtype.__setitem__(2, 99), E_UNSUPPORTED, "dtype")
+    _still_matches(interp, src, "elementwise_kernel", kw, {"out_add_ptr": True, "out_select_ptr": True, "out_ext_add_ptr": True})
+    interp.close()
