@@ -297,12 +297,13 @@ typedef struct {
     ktb_rp_scalar scal[KTB_RP_MAX_SCAL];
     ktb_rp_phase out;                        /* op unused */
     ktb_rp_side side[KTB_RP_MAX_SIDE];
-    int32_t aligned;                         /* read by ktb_launch_row_program_any: 1: every offset, row and block stride of the
-                                                operand and output tiles is a multiple of 8 elements */
+    int32_t aligned;                         /* 1: every offset, row and block stride of the operand and output tiles is a multiple
+                                                of 8 elements (rows then move as 16-byte copies; always so for
+                                                ktb_launch_row_program, where 0 only keeps it from those copies) */
     int32_t reserved;
 } ktb_rowprog_args;
 int ktb_launch_row_program(ktb_ctx* ctx, const ktb_rowprog_args* args);
-/* The same for rows of any length in [1, 16384]; offsets and strides are any number of elements. */
+/* The same for rows of any length in [1, 16384]; offsets and strides are any number of elements unless `aligned` is set. */
 int ktb_launch_row_program_any(ktb_ctx* ctx, const ktb_rowprog_args* args);
 
 /* ---- row gather / ordered row scatter ---------------------------------------------

@@ -791,7 +791,8 @@ static int rp_check_program(ktb_ctx* ctx, const ktb_vm_program& p, int n_in, boo
     return KTB_OK;
 }
 
-// What both launchers check; `any`: rows of any length, at any element.
+// What both launchers check; `any`: rows of any length, at any element unless the block says `aligned` (which sends rows
+// to 16-byte copies: strides that contradict it must not get there).
 static int rp_check_args(ktb_ctx* ctx, const ktb_rowprog_args& a, bool any) {
     if (a.n_in < 1 || a.n_in > KTB_VM_MAX_IN || a.n_red < 0 || a.n_red > KTB_RP_MAX_RED || a.n_scal < 0 ||
         a.n_scal > KTB_RP_MAX_SCAL || a.n_in + a.n_scal > KTB_VM_REGS)
@@ -804,12 +805,13 @@ static int rp_check_args(ktb_ctx* ctx, const ktb_rowprog_args& a, bool any) {
     for (int p = 0; p < a.n_red; ++p) any_blocked = any_blocked || a.red[p].blocked;
     if (a.n_blocks < 1 || a.n_blocks > 4096 || (!any_blocked && a.n_blocks != 1) || (a.out.blocked && a.out_per_row))
         return ktb_fail(ctx, KTB_E_ARG, "row_program", "bad column-block count");
-    for (int k = 0; !any && any_blocked && k <= a.n_in; ++k)
+    const bool aligned = !any || a.aligned;
+    for (int k = 0; aligned && any_blocked && k <= a.n_in; ++k)
         if (a.blk_stride[k] % 8) return ktb_fail(ctx, KTB_E_UNSUPPORTED, "row_program", "block strides must be multiples of 8 elements");
     for (int k = 0; k <= a.n_in; ++k) {
         if (a.dtype[k] != KTB_F16 && a.dtype[k] != KTB_F32)
             return ktb_fail(ctx, KTB_E_UNSUPPORTED, "row_program", "operand dtype must be f16 or f32");
-        if (!any && a.row_stride[k] % 8 && !(k == a.n_in && a.out_per_row))
+        if (aligned && a.row_stride[k] % 8 && !(k == a.n_in && a.out_per_row))
             return ktb_fail(ctx, KTB_E_UNSUPPORTED, "row_program", "row strides must be multiples of 8 elements");
     }
     if (a.n_side < 0 || a.n_side > KTB_RP_MAX_SIDE || (a.n_side && a.out_per_row))

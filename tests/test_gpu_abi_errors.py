@@ -304,3 +304,58 @@ def test_elementwise_launcher_for_several_stores_refuses_bad_programs(build_lib)
     broken(lambda a: a.dtype.__setitem__(2, 99), E_UNSUPPORTED, "dtype")
     _still_matches(interp, src, "elementwise_kernel", kw, {"out_add_ptr": True, "out_select_ptr": True, "out_ext_add_ptr": True})
     interp.close()
+
+
+def test_row_launchers_for_any_length_refuse_bad_rows(build_lib):
+    """(Strides that contradict `aligned` would be copied from between 16-byte boundaries: refused on the host.)"""
+    rng = np.random.default_rng(9)
+    rows, cols = 24, 1000
+    kw = dict(x_ptr=rng.standard_normal((rows, cols)).astype(np.float16), w_ptr=rng.standard_normal(cols).astype(np.float16),
+              y_ptr=np.zeros((rows, cols), np.float16), rstd_ptr=np.zeros(rows, np.float32))
+    src = K.rmsnorm_rows(rows, cols, 4, 2, weight=True)
+    interp, sess = _session(src, "rmsnorm_kernel", kw)
+    dev, stmt = sess.dev, _only(sess, "row_program")
+    launch = dev.lib.ktb_launch_row_program_any
+    assert stmt.symbol == "ktb_launch_row_program_any" and stmt.args.aligned == 1
+
+    def broken(change, code, *words):
+        a = _copy(stmt.args, sess.arena)
+        change(a)
+        _refused(dev, launch, a, code, "row_program", *words)
+    for k in (0, stmt.args.n_in):
+        broken(lambda a: a.row_stride.__setitem__(k, cols + 4), E_UNSUPPORTED, "multiples of 8")
+    broken(lambda a: setattr(a, "cols", 16385), E_UNSUPPORTED, "16384")
+    broken(lambda a: setattr(a, "cols", 0), E_UNSUPPORTED, "16384")
+    broken(lambda a: setattr(a, "n_blocks", 2), E_ARG, "column-block")
+    broken(lambda a: a.dtype.__setitem__(0, 9), E_UNSUPPORTED, "dtype")
+    _still_matches(interp, src, "rmsnorm_kernel", kw, {"y_ptr": True, "rstd_ptr": True})
+    interp.close()
+    # column blocks that contradict it
+    rc = (6, 3 * 256)
+    kw = dict(X=rng.standard_normal(rc).astype(np.float16), Y=np.zeros(rc, np.float16), W=rng.standard_normal(rc).astype(np.float16),
+              B=rng.standard_normal(rc).astype(np.float16), Mean=np.zeros(6, np.float16), Rstd=np.zeros(6, np.float16), N=rc[1],
+              eps=np.float16(1e-5), BLOCK_SIZE=256)
+    src = K.layernorm_blocked(*rc, 256, 3)
+    interp, sess = _session(src, "_layer_norm_fwd_fused", kw)
+    dev, stmt = sess.dev, _only(sess, "row_program")
+    assert stmt.args.aligned == 1 and stmt.args.n_blocks == 3
+    a = _copy(stmt.args, sess.arena)
+    a.blk_stride[0] = 252
+    _refused(dev, launch, a, E_UNSUPPORTED, "row_program", "block strides")
+    _still_matches(interp, src, "_layer_norm_fwd_fused", kw, {"Y": True, "Mean": True, "Rstd": True})
+    interp.close()
+    # softmax rows
+    x = rng.standard_normal((24, 1000)).astype(np.float16)
+    kw = dict(output_ptr=np.zeros_like(x), input_ptr=x)
+    src = K.softmax_rows(24, 1000, 4, 2)
+    interp, sess = _session(src, "softmax_kernel", kw)
+    dev, stmt = sess.dev, _only(sess, "row_softmax")
+    launch = dev.lib.ktb_launch_row_softmax_any
+    for change, words in ((dict(cols=16385), "16384"), (dict(cols=0), "16384"), (dict(cols=16384, aligned=0), "16377"), (dict(in_dtype=7), "dtype"),
+                          (dict(n_items=1 << 31, rows_per_item=1), "2^31")):
+        a = _copy(stmt.args, sess.arena)
+        for k, v in change.items():
+            setattr(a, k, v)
+        _refused(dev, launch, a, E_UNSUPPORTED, "row_softmax_any", words)
+    _still_matches(interp, src, "softmax_kernel", kw, {"output_ptr": False})
+    interp.close()
