@@ -473,10 +473,12 @@ typedef struct {
        the same for every launch that shares it (a launch over some of the heads, say) and no less than the launch has;
        0: those of this launch.  Launches that share scratch must be ordered.  0 / NULL: one CTA per query head, as for
        any number of rows.  steps: 64-position steps that the pieces are cut from, 0: those that the launch's rows see (a
-       launch over some rows of a statement names the whole's, so that a row is summed in the same pieces). */
+       launch over some rows of a statement names the whole's, so that a row is summed in the same pieces).
+       scratch_bytes: what dev_scratch holds; less than the above is refused. */
     int32_t splits, scratch_heads;
     void* dev_scratch;
     int32_t steps, reserved;
+    int64_t scratch_bytes;
 } ktb_attn_args;
 int ktb_launch_attention_fwd(ktb_ctx* ctx, const ktb_attn_args* args);
 

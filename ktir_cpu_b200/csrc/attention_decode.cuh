@@ -46,6 +46,10 @@ static __device__ __forceinline__ void ad_ldm4t(uint32_t addr, uint32_t (&r)[4])
 // (max, sum).  The counters outlive a launch, so where they end depends on the heads that the scratch is laid out for
 // and not on those of the launch: parts of a statement share one scratch with the whole of it.
 static __host__ __device__ __forceinline__ size_t ad_counter_bytes(int heads) { return ((size_t)heads * 32 + 255) & ~(size_t)255; }
+static int64_t ad_scratch_bytes(const ktb_attn_args& a, int group) {
+    const int heads = a.heads / group;
+    return (int64_t)ad_counter_bytes(a.scratch_heads ? a.scratch_heads : heads) + (int64_t)heads * a.splits * a.seq_q * group * 32 * 24;
+}
 
 template <int MT>                        // tiles of 16 query rows
 __global__ void __launch_bounds__(AD_THREADS, 1)

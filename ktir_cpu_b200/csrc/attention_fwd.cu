@@ -622,8 +622,11 @@ extern "C" int ktb_launch_attention_fwd(ktb_ctx* ctx, const ktb_attn_args* args)
     // Up to 32 query rows per K/V head, and pieces asked for with scratch to merge them in: the decode kernel.  (Where it is
     // the faster one: decode_pieces in lower_attn.py, which chooses the pieces.)
     const bool decode = a.splits > 0 && a.dev_scratch && a.heads % kvg == 0 && (int64_t)a.seq_q * kvg <= AD_MAX_ROWS;
+    if (a.splits < 0) return ktb_fail(ctx, KTB_E_ARG, "attention_fwd", "a negative number of pieces");
     if (decode && a.scratch_heads != 0 && a.scratch_heads < a.heads / kvg)
         return ktb_fail(ctx, KTB_E_ARG, "attention_fwd", "scratch laid out for fewer K/V heads than the launch has");
+    if (decode && (a.splits > (1 << 20) || (int64_t)(a.heads / kvg) * a.splits > (1 << 24) || a.scratch_bytes < ad_scratch_bytes(a, kvg)))
+        return ktb_fail(ctx, KTB_E_ARG, "attention_fwd", "scratch too small for the pieces");
     const uint32_t box_rows = decode && a.page > AD_ROWS ? AD_ROWS : (uint32_t)a.page;
     for (int which = 0; which < 2; ++which) {
         const uint64_t dims[4] = {AT_D, (uint64_t)((a.heads + kvg - 1) / kvg), (uint64_t)a.page, (uint64_t)a.n_pages_total};

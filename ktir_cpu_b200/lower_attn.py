@@ -364,11 +364,12 @@ class AttentionStatement(Statement):
         for ptr in self.device_arrays:
             dev.free(ptr)
         self.device_arrays, a.dev_scratch = [], None
-        a.splits, a.steps, a.scratch_heads = splits, steps, 0
+        a.splits, a.steps, a.scratch_heads, a.scratch_bytes = splits, steps, 0, 0
         if splits:
             a.scratch_heads = kv_heads = a.heads // a.kv_group   # (parts keep it: their counters are the whole's)
             counters = (kv_heads * 8 * 4 + 255) // 256 * 256
-            a.dev_scratch = dev.alloc(counters + kv_heads * splits * a.seq_q * a.kv_group * 32 * 24)
+            a.scratch_bytes = counters + kv_heads * splits * a.seq_q * a.kv_group * 32 * 24
+            a.dev_scratch = dev.alloc(a.scratch_bytes)
             dev.memset(a.dev_scratch, 0, counters)
             dev.sync()                            # (the context may be moved to another stream before the first run)
             self.device_arrays = [a.dev_scratch]

@@ -131,7 +131,7 @@ class AttnArgs(C.Structure):
                 ("kv_page_stride", C.c_int64), ("kv_row_stride", C.c_int64), ("kv_head_stride", C.c_int64),
                 ("scale", C.c_float), ("m_init", C.c_float), ("l_init", C.c_float), ("kv_group", C.c_int32),
                 ("splits", C.c_int32), ("scratch_heads", C.c_int32), ("dev_scratch", C.c_void_p),
-                ("steps", C.c_int32), ("reserved", C.c_int32)]
+                ("steps", C.c_int32), ("reserved", C.c_int32), ("scratch_bytes", C.c_int64)]
 
 
 G_MAXDIM = 6

@@ -359,3 +359,20 @@ def test_row_launchers_for_any_length_refuse_bad_rows(build_lib):
         _refused(dev, launch, a, E_UNSUPPORTED, "row_softmax_any", words)
     _still_matches(interp, src, "softmax_kernel", kw, {"output_ptr": False})
     interp.close()
+
+
+def test_attention_launcher_refuses_scratch_that_does_not_hold_the_pieces(build_lib):
+    from test_gpu_attention_decode import _case
+    src, kw = _case(1, 2000, 16, 4, 64)
+    interp, sess = _session(src, "paged_attention_kernel", kw)
+    dev, stmt = sess.dev, _only(sess, "attention_fwd")
+    assert stmt.args.splits == 32 and stmt.args.steps == 32 and stmt.args.scratch_heads == 4
+    for change, words in ((dict(scratch_bytes=stmt.args.scratch_bytes - 1), "too small"), (dict(splits=36), "too small"), (dict(splits=-4), "negative"),
+                          (dict(splits=1 << 30), "too small"), (dict(scratch_heads=3), "fewer K/V heads"), (dict(scratch_heads=9), "too small"),
+                          (dict(steps=31), "steps"), (dict(steps=33), "steps")):
+        a = _copy(stmt.args, sess.arena)
+        for k, v in change.items():
+            setattr(a, k, v)
+        _refused(dev, dev.lib.ktb_launch_attention_fwd, a, E_ARG, "attention_fwd", words)
+    _still_matches(interp, src, "paged_attention_kernel", kw, {"output_ptr": False})
+    interp.close()
