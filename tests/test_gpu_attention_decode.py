@@ -203,3 +203,60 @@ def test_shards_give_the_bits_of_the_whole(tokens, before, heads, kv_heads, q, w
     (200, 64, 8, 32, 4, 32), (200, 64, 8, 264, 33, 4), (200, 64, 8, 272, 34, 2), (200, 64, 8, 592, 74, 2), (200, 64, 8, 600, 75, 1), (200, 64, 33, 33, 1, 0)])
 def test_pieces_of_a_context(steps, page, rows, heads, kv_heads, pieces):
     assert decode_pieces(steps, page, rows, heads, kv_heads) == pieces
+
+
+def _against_oracle(src, kw, one_plan=True):
+    gpu = KTIRInterpreter()
+    gpu.load(src)
+    got = gpu.execute_function("paged_attention_kernel", **kw)["output_ptr"]
+    st, = [s for sess in gpu._sessions.values() for s in sess.plan.statements]
+    assert st.kind == "attention_fwd" and st.args.splits >= 1
+    gpu.close()
+    ora = OracleInterpreter()
+    ora.load(src)
+    with np.errstate(all="ignore"):
+        want = ora.execute_function("paged_attention_kernel", **kw)["output_ptr"]
+    np.testing.assert_allclose(got.astype(np.float32), want.astype(np.float32), rtol=1e-2, atol=2e-3)
+    return st
+
+
+# one piece, a cluster, several clusters with the merge through scratch
+FORMS = [(1, 63, 4, 2, 64), (3, 509, 6, 3, 128), (8, 1016, 4, 1, 32), (32, 992, 1, 1, 64)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tokens,before,heads,kv_heads,page", FORMS)
+def test_decode_without_a_mask(tokens, before, heads, kv_heads, page, build_lib):
+    """Every row sees every position."""
+    src, kw = _case(tokens, before, heads, kv_heads, page)
+    assert (tokens + before) % page == 0
+    for use in ("ins(%masked :", "ins(%masked,"):
+        assert src.count(use) == 1
+        src = src.replace(use, use.replace("%masked", "%sc"))
+    assert not _against_oracle(src, kw).args.causal
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m_init,l_init", [(0.5, 3.0), (-2.0, 0.0), (6.0, 1.0)])
+@pytest.mark.parametrize("tokens,before,heads,kv_heads,page", FORMS)
+def test_decode_with_initial_maximum_and_sum(tokens, before, heads, kv_heads, page, m_init, l_init, build_lib):
+    """A running maximum and sum that start at finite values (a position without a value): once per row, however many pieces."""
+    src, kw = _case(tokens, before, heads, kv_heads, page)
+    for name, old, value in (("m_init", "ninf", m_init), ("l_init", "one", l_init)):
+        assert src.count(f"%{name} = tensor.splat %{old} ") == 1
+        src = src.replace(f"%{name} = tensor.splat %{old} ", f"%{name}_v = arith.constant {value} : f32\n    %{name} = tensor.splat %{name}_v ")
+    a = _against_oracle(src, kw).args
+    assert (a.m_init, a.l_init) == (m_init, l_init)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("which,value", [("key_cache_ptr", np.nan), ("key_cache_ptr", np.inf), ("value_cache_ptr", np.nan), ("value_cache_ptr", -np.inf)])
+@pytest.mark.parametrize("tokens,before,heads,kv_heads,page", FORMS)
+def test_decode_of_special_values(tokens, before, heads, kv_heads, page, which, value, build_lib):
+    """One element of one visible position of K/V head 0: NaN reaches every row that sees it, an infinite score makes NaN
+    (or vanishes, where it is negative), an infinite value stays."""
+    src, kw = _case(tokens, before, heads, kv_heads, page)
+    pos = before // 2
+    kw[which] = kw[which].copy()
+    kw[which][kw["block_tables_ptr"][0, pos // page], pos % page, 0, 5] = value
+    _against_oracle(src, kw)

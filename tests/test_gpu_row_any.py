@@ -1,4 +1,6 @@
 """Row kernels for rows of any length and alignment (``ktb_launch_row_softmax_any``) against the oracle."""
+import re
+
 import numpy as np
 import pytest
 
@@ -157,3 +159,81 @@ def test_softmax_with_initial_values(cols, max_init, sum_init, low, high, build_
     got, want, kinds, symbols = _both(src, "softmax_kernel", dict(output_ptr=np.zeros_like(x), input_ptr=x))
     assert kinds == ["row_softmax"] and symbols == ["ktb_launch_row_softmax_any"]
     np.testing.assert_allclose(got["output_ptr"].astype(np.float32), want["output_ptr"].astype(np.float32), rtol=2e-3, atol=2e-6)
+
+
+def _f32(src):
+    """The kernel over f32 tiles: no casts between the two types."""
+    src = src.replace("f16", "f32")
+    for name, of in re.findall(r"^ *(%\w+) = arith\.(?:extf|truncf) (%\w+) :.*\n", src, re.M):
+        src = re.sub(rf"^ *{name} = arith\.(?:extf|truncf) {of} :.*\n", "", src, flags=re.M)
+        src = re.sub(rf"{name}\b", of, src)
+    return src
+
+
+def _special_rows(rows, cols, dt):
+    """NaN at one place and everywhere, infinities of either sign at one place and everywhere, the lowest value everywhere
+    and in all places but one."""
+    x = (np.random.default_rng(cols).standard_normal((rows, cols)) * 2).astype(dt)
+    x[0, cols // 2], x[1] = np.nan, np.nan
+    x[2, 0], x[3], x[4, 1:], x[5, cols - 1], x[6] = -np.inf, -np.inf, -np.inf, np.inf, np.inf
+    x[7], x[8, 1:] = np.finfo(dt).min, np.finfo(dt).min
+    x[9, 0], x[9, 1] = np.nan, np.inf
+    return x
+
+
+@pytest.mark.parametrize("maxop", ["maximumf", "maxnumf"])
+@pytest.mark.parametrize("form", ["f16 rows, f32 statistics", "f16 arithmetic", "f32 rows"])
+@pytest.mark.parametrize("cols", [5, 250, 3001])
+def test_softmax_of_special_values(cols, form, maxop, build_lib):
+    """f16 results: 2e-3 and 1e-2 as above.  f32 results: the sum in another order (cols 2^-24 at most) and two steps of the
+    device's and of NumPy's exp (2^-21)."""
+    x = _special_rows(12, cols, np.float32 if form == "f32 rows" else np.float16)
+    src = K.softmax_rows(12, cols, 4, 1, form != "f16 arithmetic").replace("arith.maximumf", "arith." + maxop)
+    if form == "f32 rows":
+        src = _f32(src)
+    with np.errstate(all="ignore"):
+        got, want, kinds, symbols = _both(src, "softmax_kernel", dict(output_ptr=np.full_like(x, 9), input_ptr=x))
+    assert kinds == ["row_softmax"] and symbols == ["ktb_launch_row_softmax_any"]
+    rtol, atol = {"f32 rows": (2.0 ** -21 + cols * 2.0 ** -24, 0), "f16 arithmetic": (1e-2, 1e-5)}.get(form, (2e-3, 2e-6))
+    np.testing.assert_allclose(got["output_ptr"].astype(np.float32), want["output_ptr"].astype(np.float32), rtol=rtol, atol=atol)
+
+
+@pytest.mark.parametrize("form", ["f16 rows, f32 statistics", "f16 arithmetic", "f32 rows"])
+@pytest.mark.parametrize("rows,cols", [(64, 250), (40, 2049), (8, 9001)])
+def test_softmax_in_place(rows, cols, form, build_lib):
+    x = np.random.default_rng(cols).standard_normal((rows, cols)).astype(np.float32 if form == "f32 rows" else np.float16)
+    src = K.softmax_rows(rows, cols, 4, 2, form != "f16 arithmetic").replace("construct_memory_view %output_ptr", "construct_memory_view %input_ptr")
+    if form == "f32 rows":
+        src = _f32(src)
+    got, want, kinds, symbols = _both(src, "softmax_kernel", dict(output_ptr=np.full_like(x, 9), input_ptr=x))
+    assert kinds == ["row_softmax"] and symbols == ["ktb_launch_row_softmax_any"]
+    rtol, atol = {"f32 rows": (2.0 ** -21 + cols * 2.0 ** -24, 0), "f16 arithmetic": (1e-2, 1e-5)}.get(form, (2e-3, 2e-6))
+    np.testing.assert_allclose(got["input_ptr"].astype(np.float32), want["input_ptr"].astype(np.float32), rtol=rtol, atol=atol)
+    np.testing.assert_array_equal(got["output_ptr"], 9)
+
+
+# odd lengths, whole vectors, whole eighths (the wide first fold), one warp and several
+F32_ROWS = [(24, 261), (12, 1000), (20, 1024), (6, 5001), (3, 9984)]
+
+
+@pytest.mark.parametrize("rows,cols", F32_ROWS)
+def test_normalisations_of_f32_tiles(rows, cols, build_lib):
+    """The same kernel over f32 rows: plain row norm, layer norm and column blocks, the oracle's bits."""
+    rng = np.random.default_rng(cols)
+    f = lambda *s: rng.standard_normal(s, dtype=np.float32)     # noqa: E731
+    x, w, b = f(rows, cols), f(cols), f(cols)
+    cores = next(c for c in (4, 3, 2) if rows % c == 0)
+    got, want, kinds, symbols = _both(_f32(K.rmsnorm_rows(rows, cols, cores, 1, weight=True)), "rmsnorm_kernel",
+                                      dict(x_ptr=x, w_ptr=w, y_ptr=np.zeros_like(x), rstd_ptr=np.zeros(rows, np.float32)))
+    assert kinds == ["row_program"]
+    _bits(got, want, ("y_ptr", "rstd_ptr"))
+    got, want, kinds, symbols = _both(_f32(K.layernorm_rows(rows, cols, cores)), "layernorm_kernel",
+                                      dict(x_ptr=x, w_ptr=w, b_ptr=b, y_ptr=np.zeros_like(x), mean_ptr=np.zeros(rows, np.float32)))
+    assert kinds == ["row_program"]
+    _bits(got, want, ("y_ptr", "mean_ptr"))
+    rc = (rows, 3 * (cols // 3))
+    kw = dict(X=f(*rc), Y=np.zeros(rc, np.float32), W=f(*rc), B=f(*rc), Mean=np.zeros(rows, np.float32), Rstd=np.zeros(rows, np.float32), N=rc[1],
+              eps=np.float32(1e-5), BLOCK_SIZE=cols // 3)
+    got, want, kinds, symbols = _both(_f32(K.layernorm_blocked(*rc, cols // 3, cores)), "_layer_norm_fwd_fused", kw)
+    assert kinds == ["row_program"]
+    _bits(got, want, ("Mean", "Rstd", "Y"))
