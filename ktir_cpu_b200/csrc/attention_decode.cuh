@@ -12,7 +12,7 @@
 // merged through shared memory, then the pieces of a cluster through distributed shared memory, each CTA taking a slice
 // of the rows.  With several clusters per head a CTA leaves its slice in scratch and the last one to finish that slice
 // (a counter that wraps to zero by itself) merges it.  No CTA waits for another outside its cluster.
-// 1 token, 64 / 8 heads, 8192 positions f16 (33.5 MB): 16.0 us (5.2 at the measured copy rate), 88 with
+// 1 token, 64 / 8 heads, 8192 positions f16 (33.5 MB): 15.8 us (5.1 at the measured copy rate), 88 with
 // a CTA per query head; 2 tokens, 128 / 32 heads, 16002 positions (264 MB): 47.2 (40.9), 169 before.  Measured: clusters of
 // 8 do not all fit at once (26 us), of 2 leave more to the last merge (22.6 against 18.1 at 32 rows), two CTAs per SM
 // with half the ring each 22.0.

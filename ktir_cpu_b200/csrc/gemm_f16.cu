@@ -376,8 +376,8 @@ ktb_gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
 // ktb_gemm_f16_kernel; A tiles hold no more rows than the matrix has (the accumulator rows beyond are never read).  The
 // f32 partial tiles meet in shared memory: every CTA adds up a 1 / S-th of the rows over its cluster, range after range,
 // so a sum's order depends on S and K alone, not on the tile that it falls into.
-// Bound by the chain load -> MMA -> exchange of one tile, next to reading B.  f16 [64, 2880] x [2880, 5760]: 14.6 us
-// (5.3 at the measured copy rate), 20.6 on 23 tiles of 256 columns; [16, 4096] x [4096, 512]: 10.3, 24.6 before.
+// Bound by the chain load -> MMA -> exchange of one tile, next to reading B.  f16 [64, 2880] x [2880, 5760]: 14.4 us
+// (5.2 at the measured copy rate), 20.5 on 23 tiles of 256 columns; [16, 4096] x [4096, 512]: 10.3, 24.6 before.
 template <int BN>
 struct GemmFew {
     static constexpr int STAGES = BN == 64 ? 8 : 6;

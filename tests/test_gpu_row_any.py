@@ -1,4 +1,5 @@
-"""Row kernels for rows of any length and alignment (``ktb_launch_row_softmax_any``) against the oracle."""
+"""Row kernels for rows of any length and alignment (``ktb_launch_row_softmax_any``, ``ktb_launch_row_program_any``) against
+the oracle."""
 import re
 
 import numpy as np
@@ -96,8 +97,8 @@ def test_layernorm_rows_of_any_length(rows, cols, cores, build_lib):
 @pytest.mark.parametrize("rows,block,blocks,cores", [(11, 53, 7, 3), (37, 1024, 3, 32), (9, 361, 6, 4), (12, 256, 5, 5), (5, 1500, 8, 2),
                                                      (6, 448, 1, 3), (3, 2048, 8, 2)])
 def test_column_blocked_layernorm_of_any_length(rows, block, blocks, cores, build_lib):
-    """f16 throughout: every add of the block accumulation and of the fold rounds, in the reference's order.  (One block:
-    the block loop leaves no accumulator to recognise and Mean / Rstd / Y are statements of their own.)"""
+    """f16 throughout: every add of the block accumulation and of the fold rounds, in the reference's order.  (One
+    block too: the loop of one trip is a chain of one term, and Mean and Rstd leave with the launch.)"""
     rng = np.random.default_rng(block)
     rc = (rows, block * blocks)
     kw = dict(X=rng.standard_normal(rc).astype(np.float16), Y=np.zeros(rc, np.float16), W=rng.standard_normal(rc).astype(np.float16),
